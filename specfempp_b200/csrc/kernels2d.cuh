@@ -52,6 +52,41 @@ constexpr int NP = 25;
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
+// Programmatic dependent launch.  The single-shot owner-computes step is a
+// chain of short kernels (element kernel, late receivers, point update), so
+// the launch gap and each kernel's first static loads are a large part of a
+// step on a small mesh.  Each kernel of the chain may start while its
+// predecessor drains: it issues the loads of data no kernel of the step
+// writes (indices, geometry, material, M^-1; the update also u and v, which
+// only updates write), then waits in pdl_wait for the predecessor's grid to
+// complete, and only then lets its own successor start.  That order matters:
+// a grid that has started has its predecessor's predecessor complete.  Data
+// written by the step's kernels is read after the wait with ld_dep, which the
+// compiler may neither hoist over the wait nor turn into a read-only-cache
+// load.  In a launch without the attribute both calls do nothing.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ float ld_dep(const float *p) {
+  float x;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(p) : "memory");
+  return x;
+}
+__device__ __forceinline__ int ld_dep(const int *p) {
+  int x;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+  return x;
+}
+__device__ __forceinline__ float2 ld_dep2(const float *p) {
+  float2 x;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "l"(p) : "memory");
+  return x;
+}
+__device__ __forceinline__ float4 ld_dep4(const float *p) {
+  float4 x;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "l"(p) : "memory");
+  return x;
+}
+
 struct Quad {
   float hp[NP];    // hp[i*5+j] = l'_j(xi_i)
   float hpw[NP];   // hp[l*5+i] * w[l]
@@ -81,8 +116,14 @@ struct MedArgs {
   int nblocks;     // blocks of this medium in the launch
 };
 
+struct RecArgs;
+
 struct StiffArgs {
   MedArgs el, ac;
+  // receivers that read only the step's displacement, taken by the launch's
+  // first rec_blocks blocks, one warp each: acoustic ones first
+  const RecArgs *rec_ac, *rec_el;
+  int nrec_ac, nrec_el, rec_blocks;
   const int *__restrict__ src_next;
   const float *__restrict__ src_arr;   // [nsrc][2][25]
   const float *__restrict__ src_arr2;  // poroelastic fluid rows [nsrc][2][25] (else null)
@@ -134,9 +175,14 @@ __device__ __forceinline__ void elastic_block(const StiffArgs &S, const MedArgs 
   const float xix = __ldg(A.xix + p), xiz = __ldg(A.xiz + p), gax = __ldg(A.gax + p),
               gaz = __ldg(A.gaz + p), jac = __ldg(A.jac + p);
   const float c0 = __ldg(A.prop0 + p), mu = __ldg(A.prop1 + p);
+  // the slot with the other static loads where the register cap leaves room
+  constexpr bool SLOT_EARLY = LOCAL && EK <= 2;
+  const int sl0 = SLOT_EARLY ? __ldg(A.slot + p) : 0;
+  pdl_wait();
+  pdl_release();
   float uu[NC], acc[NC];
   if (NC == 4) {
-    const float4 t = act ? reinterpret_cast<const float4 *>(A.u)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 t = act ? ld_dep4(A.u + size_t(g) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     uu[0] = t.x; uu[1 % NC] = t.y; uu[2 % NC] = t.z; uu[3 % NC] = t.w;
     if (!LOCAL) {
       const float4 r = act ? reinterpret_cast<const float4 *>(A.accum)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -145,18 +191,18 @@ __device__ __forceinline__ void elastic_block(const StiffArgs &S, const MedArgs 
   } else if (NC == 3) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      uu[c] = act ? A.u[size_t(g) * 3 + c] : 0.f;
+      uu[c] = act ? ld_dep(A.u + size_t(g) * 3 + c) : 0.f;
       if (!LOCAL) acc[c] = act ? A.accum[size_t(g) * 3 + c] : 0.f;
     }
   } else if (NC == 2) {
-    const float2 t = act ? reinterpret_cast<const float2 *>(A.u)[g] : make_float2(0.f, 0.f);
+    const float2 t = act ? ld_dep2(A.u + size_t(g) * 2) : make_float2(0.f, 0.f);
     uu[0] = t.x; uu[NC - 1] = t.y;
     if (!LOCAL) {
       const float2 r = act ? reinterpret_cast<const float2 *>(A.accum)[g] : make_float2(0.f, 0.f);
       acc[0] = r.x; acc[NC - 1] = r.y;
     }
   } else {
-    uu[0] = act ? A.u[g] : 0.f;
+    uu[0] = act ? ld_dep(A.u + g) : 0.f;
     if (!LOCAL) acc[0] = act ? A.accum[g] : 0.f;
   }
   const int bs = act ? __ldg(A.bc_slot + e) : -1;
@@ -291,7 +337,7 @@ __device__ __forceinline__ void elastic_block(const StiffArgs &S, const MedArgs 
   if (EK == 3) a[NC - 1] -= (csxz - cszx) * (sw[ix] * sw[iz] * jac);   // couple stress
   if (EK == 4) {
     // viscous damping of the fluid motion; factor w_x w_z |J|
-    const float4 vv = reinterpret_cast<const float4 *>(A.v)[g];
+    const float4 vv = ld_dep4(A.v + size_t(g) * 4);
     const float fac = sw[ix] * sw[iz] * jac;
     const float exx = __ldg(A.prop6 + p), exz = __ldg(A.prop7 + p), ezz = __ldg(A.prop8 + p);
     const float viscx = fac * ((exx * vv.z) + (exz * vv.w));
@@ -308,7 +354,8 @@ __device__ __forceinline__ void elastic_block(const StiffArgs &S, const MedArgs 
     if (wq != 0.f) {
       const float nx = A.bc_nx[k], nz = A.bc_nz[k], j1 = A.bc_j1[k];
       if (EK == 3) {
-        const float vx = A.v[size_t(g) * 3], vz = A.v[size_t(g) * 3 + 1], vr = A.v[size_t(g) * 3 + 2];
+        const float vx = ld_dep(A.v + size_t(g) * 3), vz = ld_dep(A.v + size_t(g) * 3 + 1),
+                    vr = ld_dep(A.v + size_t(g) * 3 + 2);
         const float rvp = A.bc_imp0[k], rvs = A.bc_imp1[k];
         const float vn = vx * nx + vz * nz;
         const float fx = ((vn * nx / (j1 * j1)) * (rvp - rvs)) + vx * rvs;
@@ -317,7 +364,7 @@ __device__ __forceinline__ void elastic_block(const StiffArgs &S, const MedArgs 
         a[1] += -1.f * fz * j1 * wq;
         a[NC - 1] += -1.f * A.bc_imp2[k] * vr * j1 * wq;
       } else if (EK != 1) {
-        const float2 vv = reinterpret_cast<const float2 *>(A.v)[g];
+        const float2 vv = ld_dep2(A.v + size_t(g) * 2);
         const float rvp = A.bc_imp0[k], rvs = A.bc_imp1[k];
         const float vn = vv.x * nx + vv.y * nz;
         const float fx = ((vn * nx / (j1 * j1)) * (rvp - rvs)) + vv.x * rvs;
@@ -325,14 +372,14 @@ __device__ __forceinline__ void elastic_block(const StiffArgs &S, const MedArgs 
         a[0] += -1.f * fx * j1 * wq;
         a[NC - 1] += -1.f * fz * j1 * wq;
       } else {
-        a[0] += -1.f * (wq * j1) * A.bc_imp1[k] * A.v[g];
+        a[0] += -1.f * (wq * j1) * A.bc_imp1[k] * ld_dep(A.v + g);
       }
     }
   }
   if (src >= 0) {
-    const int step = *S.step;
+    const int step = ld_dep(S.step);
     for (int s = src; s >= 0; s = S.src_next[s]) {
-      const float f = step < S.nstep ? S.stf[size_t(step) * S.nsrc + s] : 0.f;
+      const float f = step < S.nstep ? ld_dep(S.stf + size_t(step) * S.nsrc + s) : 0.f;
 #pragma unroll
       for (int c = 0; c < (NC < 2 ? NC : 2); ++c) a[c] += f * S.src_arr[(size_t(s) * 2 + c) * NP + q];
       if (EK == 4) {
@@ -342,7 +389,7 @@ __device__ __forceinline__ void elastic_block(const StiffArgs &S, const MedArgs 
     }
   }
   if (LOCAL) {
-    const int sl = __ldg(A.slot + p);
+    const int sl = SLOT_EARLY ? sl0 : __ldg(A.slot + p);
     if (NC == 4) {
       reinterpret_cast<float4 *>(A.r)[sl] = make_float4(a[0], a[1 % NC], a[2 % NC], a[3 % NC]);
     } else if (NC == 3) {
@@ -379,7 +426,10 @@ __device__ __forceinline__ void acoustic_block(const StiffArgs &S, const MedArgs
   const float xix = __ldg(A.xix + p), xiz = __ldg(A.xiz + p), gax = __ldg(A.gax + p),
               gaz = __ldg(A.gaz + p), jac = __ldg(A.jac + p);
   const float rhoinv = __ldg(A.prop0 + p);
-  const float chi = act ? A.u[g] : 0.f;
+  const int sl = LOCAL ? __ldg(A.slot + p) : 0;
+  pdl_wait();
+  pdl_release();
+  const float chi = act ? ld_dep(A.u + g) : 0.f;
   const float acc = (act && !LOCAL) ? A.accum[g] : 0.f;
   const int bs = act ? __ldg(A.bc_slot + e) : -1;
   const int src = act ? __ldg(A.src_head + e) : -1;
@@ -408,17 +458,17 @@ __device__ __forceinline__ void acoustic_block(const StiffArgs &S, const MedArgs
   if (bs >= 0) {
     const size_t k = size_t(bs) * NP + q;
     const float wq = A.bc_w[k];
-    if (wq != 0.f) a += -1.f * (wq * A.bc_j1[k]) * A.bc_imp0[k] * A.v[g];
+    if (wq != 0.f) a += -1.f * (wq * A.bc_j1[k]) * A.bc_imp0[k] * ld_dep(A.v + g);
     a *= A.bc_keep[k];   // acoustic free surface (Dirichlet) zeroes the element term
   }
   if (src >= 0) {
-    const int step = *S.step;
+    const int step = ld_dep(S.step);
     for (int s = src; s >= 0; s = S.src_next[s]) {
-      const float f = step < S.nstep ? S.stf[size_t(step) * S.nsrc + s] : 0.f;
+      const float f = step < S.nstep ? ld_dep(S.stf + size_t(step) * S.nsrc + s) : 0.f;
       a += f * S.src_arr[(size_t(s) * 2) * NP + q];
     }
   }
-  if (LOCAL) A.r[__ldg(A.slot + p)] = a;
+  if (LOCAL) A.r[sl] = a;
   else A.accum[g] = acc + a;
 }
 
@@ -426,15 +476,34 @@ __device__ __forceinline__ void acoustic_block(const StiffArgs &S, const MedArgs
 // colour, the following ac.nblocks blocks acoustic ones.
 // occupancy held at the warp limit of an SM (64 warps): the kernel is bound
 // by memory latency, so registers may not grow past what that allows
+template <bool EARLY>
+__device__ void receiver_warp(const RecArgs &A, int i, int lane, float *sf);
+
+// The first rec_blocks blocks of an element launch: one receiver a warp.
+__device__ __noinline__ void receiver_blocks(const RecArgs *ac, const RecArgs *el, int nac, int nel, float *smem) {
+  const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_release();
+  const int i = blockIdx.x * nw + w;
+  if (w >= nw || i >= nac + nel) return;
+  if (i < nac) receiver_warp<true>(*ac, i, lane, smem + w * 3 * NP);
+  else receiver_warp<true>(*el, i - nac, lane, smem + w * 3 * NP);
+}
+
 template <int E, int EK, bool LOCAL>
 __global__ void __launch_bounds__(NP * E, 64 / ((NP * E + 31) / 32)) k_stiffness(StiffArgs S) {
   __shared__ __align__(16) unsigned char smem[sizeof(float) * NP * E * (EK == 4 ? 12 : EK == 3 ? 9 : 6)];
   __shared__ float shp[NP], shpw[NP], sw[NG];
+  const int b = int(blockIdx.x) - S.rec_blocks;
+  if (LOCAL && b < 0) {
+    receiver_blocks(S.rec_ac, S.rec_el, S.nrec_ac, S.nrec_el, reinterpret_cast<float *>(smem));
+    return;
+  }
   load_quad(S.quad, shp, shpw, sw, threadIdx.x);
-  if (int(blockIdx.x) < S.el.nblocks)
-    elastic_block<E, EK, LOCAL>(S, S.el, S.el.e0 + blockIdx.x * E, smem, shp, shpw, sw);
+  if (b < S.el.nblocks)
+    elastic_block<E, EK, LOCAL>(S, S.el, S.el.e0 + b * E, smem, shp, shpw, sw);
   else
-    acoustic_block<E, LOCAL>(S, S.ac, S.ac.e0 + (blockIdx.x - S.el.nblocks) * E, smem, shp, shpw, sw);
+    acoustic_block<E, LOCAL>(S, S.ac, S.ac.e0 + (b - S.el.nblocks) * E, smem, shp, shpw, sw);
 }
 
 // ---------------------------------------------------------------------------
@@ -673,10 +742,10 @@ struct UpdateArgs {
 __device__ __forceinline__ float coupling_entry(const UpdateArgs &A, int k, int comp) {
   const int o = A.cp_other[k];
   if (A.ncomp == 1) {  // acoustic self: n . u_elastic
-    const float2 ue = reinterpret_cast<const float2 *>(A.other)[o];
+    const float2 ue = ld_dep2(A.other + size_t(o) * 2);
     return A.cp_nx[k] * ue.x + A.cp_nz[k] * ue.y;
   }
-  const float chi_dd = A.other[o];  // elastic self: n * chi_dd
+  const float chi_dd = ld_dep(A.other + o);  // elastic self: n * chi_dd
   return (comp == 0 ? A.cp_nx[k] : A.cp_nz[k]) * chi_dd;
 }
 
@@ -769,67 +838,90 @@ __global__ void __launch_bounds__(256) k_update(UpdateArgs A) {
 // element-local contributions in increasing compute order (colour order), so
 // the sum is the colour passes' sum bit for bit; then coupling, M^-1,
 // corrector and optional predictor as k_update.  No accumulator to clear.
+//
+// The loads of a point come in two parts: what no kernel since the last
+// update writes (contribution range, u, v, M^-1) before the wait, the
+// contributions after it.
 template <int NC>
-__device__ __forceinline__ bool update_gather_point(const UpdateArgs &A, int g) {
+struct PointPre {
+  int k0, k1;
+  float u[NC], v[NC], mi[NC];
+};
+
+template <int NC>
+__device__ __forceinline__ PointPre<NC> update_point_pre(const UpdateArgs &A, int g) {
+  PointPre<NC> P;
+  P.k0 = A.inv_start[g];
+  P.k1 = A.inv_start[g + 1];
+  if (NC > 2) return P;      // u, v and M^-1 after the sum: fewer registers, more warps
+  if (NC == 2) {
+    const float2 u2 = ld_dep2(A.u + size_t(g) * 2), v2 = ld_dep2(A.v + size_t(g) * 2);
+    const float2 m2 = reinterpret_cast<const float2 *>(A.minv)[g];
+    P.u[0] = u2.x; P.u[NC - 1] = u2.y; P.v[0] = v2.x; P.v[NC - 1] = v2.y; P.mi[0] = m2.x; P.mi[NC - 1] = m2.y;
+  } else {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const size_t i = size_t(g) * NC + c;
+      P.u[c] = ld_dep(A.u + i); P.v[c] = ld_dep(A.v + i); P.mi[c] = A.minv[i];
+    }
+  }
+  return P;
+}
+
+template <int NC>
+__device__ __forceinline__ bool update_point_post(const UpdateArgs &A, int g, PointPre<NC> &P) {
   float acc[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) acc[c] = 0.f;
-  const int k1 = A.inv_start[g + 1];
-  for (int k = A.inv_start[g]; k < k1; ++k) {
+  for (int k = P.k0; k < P.k1; ++k) {
     if (NC == 2) {
-      const float2 t = reinterpret_cast<const float2 *>(A.r)[k];
+      const float2 t = ld_dep2(A.r + size_t(k) * 2);
       acc[0] = acc[0] + t.x;
       acc[NC - 1] = acc[NC - 1] + t.y;
     } else {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) acc[c] = acc[c] + A.r[size_t(k) * NC + c];
+      for (int c = 0; c < NC; ++c) acc[c] = acc[c] + ld_dep(A.r + size_t(k) * NC + c);
     }
   }
   if (g < A.niface) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[c] += coupling_term(A, g, c);
   }
-  float uu[NC], vv[NC], mi[NC];
-  if (NC == 2) {
-    const float2 u2 = reinterpret_cast<const float2 *>(A.u)[g];
-    const float2 v2 = reinterpret_cast<const float2 *>(A.v)[g];
-    const float2 m2 = reinterpret_cast<const float2 *>(A.minv)[g];
-    uu[0] = u2.x; uu[NC - 1] = u2.y; vv[0] = v2.x; vv[NC - 1] = v2.y; mi[0] = m2.x; mi[NC - 1] = m2.y;
-  } else {
+  if (NC > 2) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const size_t i = size_t(g) * NC + c;
-      uu[c] = A.u[i]; vv[c] = A.v[i]; mi[c] = A.minv[i];
+      P.u[c] = ld_dep(A.u + i); P.v[c] = ld_dep(A.v + i); P.mi[c] = A.minv[i];
     }
   }
   float a[NC];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) a[c] = __fmul_rn(acc[c], mi[c]);
+  for (int c = 0; c < NC; ++c) a[c] = __fmul_rn(acc[c], P.mi[c]);
   if (A.rec) {
     const size_t off = size_t(*A.step - A.rec->k0) * A.rec->stride;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      A.rec->u[off + size_t(g) * NC + c] = uu[c];
+      A.rec->u[off + size_t(g) * NC + c] = P.u[c];
       A.rec->a[off + size_t(g) * NC + c] = a[c];
     }
   }
   bool bad = false;
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
-    vv[c] = newmark_correct(vv[c], a[c], A.dt2);
-    if (A.predict) newmark_predict(uu[c], vv[c], a[c], A.dt, A.dt2, A.dtsq2);
-    bad |= !isfinite(uu[c]);
+    P.v[c] = newmark_correct(P.v[c], a[c], A.dt2);
+    if (A.predict) newmark_predict(P.u[c], P.v[c], a[c], A.dt, A.dt2, A.dtsq2);
+    bad |= !isfinite(P.u[c]);
   }
   if (NC == 2) {
-    if (A.predict) reinterpret_cast<float2 *>(A.u)[g] = make_float2(uu[0], uu[NC - 1]);
-    reinterpret_cast<float2 *>(A.v)[g] = make_float2(vv[0], vv[NC - 1]);
+    if (A.predict) reinterpret_cast<float2 *>(A.u)[g] = make_float2(P.u[0], P.u[NC - 1]);
+    reinterpret_cast<float2 *>(A.v)[g] = make_float2(P.v[0], P.v[NC - 1]);
     if (A.a_store) reinterpret_cast<float2 *>(A.a_store)[g] = make_float2(a[0], a[NC - 1]);
   } else {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const size_t i = size_t(g) * NC + c;
-      if (A.predict) A.u[i] = uu[c];
-      A.v[i] = vv[c];
+      if (A.predict) A.u[i] = P.u[c];
+      A.v[i] = P.v[c];
       if (A.a_store) A.a_store[i] = a[c];
     }
   }
@@ -837,12 +929,20 @@ __device__ __forceinline__ bool update_gather_point(const UpdateArgs &A, int g) 
 }
 
 template <int NC>
-__global__ void __launch_bounds__(256) k_update_gather(UpdateArgs A) {
+__global__ void __launch_bounds__(256, NC <= 2 ? 8 : 6) k_update_gather(UpdateArgs A) {
   const int npts = A.n / NC;
   const int stride = gridDim.x * blockDim.x;
   bool bad = false;
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < npts; g += stride)
-    bad |= update_gather_point<NC>(A, g);
+  int g = blockIdx.x * blockDim.x + threadIdx.x;
+  PointPre<NC> P;
+  if (g < npts) P = update_point_pre<NC>(A, g);
+  pdl_wait();
+  pdl_release();
+  while (g < npts) {
+    bad |= update_point_post<NC>(A, g, P);
+    g += stride;
+    if (g < npts) P = update_point_pre<NC>(A, g);
+  }
   if (bad) *A.flag = 1;
   if (A.advance && blockIdx.x == 0 && threadIdx.x == 0) *A.step += 1;
 }
@@ -857,17 +957,33 @@ __global__ void __launch_bounds__(256) k_update_gather(UpdateArgs A) {
 // launch would, before this thread overwrites the displacement) and then
 // itself (reading the chi_dd it has just stored).  Same arithmetic as the two
 // launches: equal bits.
-__global__ void __launch_bounds__(256) k_update_coupled(UpdateArgs El, UpdateArgs Ac) {
-  const int nel = El.n / 2, nac = Ac.n;
+__global__ void __launch_bounds__(256, 6) k_update_coupled(UpdateArgs El, UpdateArgs Ac) {
+  const int nel = El.n / 2, nac = Ac.n, n = nel + nac - Ac.niface;
   const int stride = gridDim.x * blockDim.x;
   bool bad = false;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nel + nac - Ac.niface; t += stride) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  PointPre<2> P;
+  PointPre<1> Q;
+  auto pre = [&]() {
+    if (t < nel) P = update_point_pre<2>(El, t);
+    else if (t < n) Q = update_point_pre<1>(Ac, Ac.niface + (t - nel));
+  };
+  pre();
+  pdl_wait();
+  pdl_release();
+  while (t < n) {
     if (t < nel) {
-      if (t < El.niface) bad |= update_gather_point<1>(Ac, El.cp_other[t]);
-      bad |= update_gather_point<2>(El, t);
+      if (t < El.niface) {
+        const int o = El.cp_other[t];
+        Q = update_point_pre<1>(Ac, o);
+        bad |= update_point_post<1>(Ac, o, Q);
+      }
+      bad |= update_point_post<2>(El, t, P);
     } else {
-      bad |= update_gather_point<1>(Ac, Ac.niface + (t - nel));
+      bad |= update_point_post<1>(Ac, Ac.niface + (t - nel), Q);
     }
+    t += stride;
+    pre();
   }
   if (bad) *El.flag = 1;
   if (El.advance && blockIdx.x == 0 && threadIdx.x == 0) *El.step += 1;
@@ -955,7 +1071,7 @@ __device__ __forceinline__ float rec_accel(const RecArgs &A, int g, int c) {
   if (A.cpl.inv_start) {   // owner-computes: gather in colour order
     acc = 0.f;
     for (int j = A.cpl.inv_start[g]; j < A.cpl.inv_start[g + 1]; ++j)
-      acc = acc + A.cpl.r[size_t(j) * A.ncomp + c];
+      acc = acc + ld_dep(A.cpl.r + size_t(j) * A.ncomp + c);
   } else {
     acc = A.accum[k];
   }
@@ -966,18 +1082,21 @@ __device__ __forceinline__ float rec_accel(const RecArgs &A, int g, int c) {
 // One warp per receiver of one medium; runs before that medium's update, so
 // it reconstructs the corrected velocity and the new acceleration from the
 // accumulator (plus the coupling term on interface points).
-__global__ void __launch_bounds__(32) k_receivers(RecArgs A) {
-  __shared__ float sf[3][NP];
+// EARLY: types that read only the displacement, taken inside the element
+// launch (whose other blocks are writing the contributions).  sf: 3 x 25
+// floats of the warp.
+template <bool EARLY>
+__device__ void receiver_warp(const RecArgs &A, int i, int lane, float *sfp) {
+  float (*sf)[NP] = reinterpret_cast<float (*)[NP]>(sfp);
   int isig = A.isig_fixed;
   if (isig < 0) {
-    const int step = *A.step;
+    const int step = ld_dep(A.step);
     if (step % A.nsb != 0) return;
     isig = step / A.nsb;
   }
   if (isig >= A.nsig) return;
-  const int r = A.rec_list[blockIdx.x];
+  const int r = A.rec_list[i];
   const int ce = A.rec_elem[r];
-  const int lane = threadIdx.x;
   const bool on = lane < NP;
   const int q = on ? lane : 0;
   const size_t p = size_t(ce) * NP + q;
@@ -1002,10 +1121,10 @@ __global__ void __launch_bounds__(32) k_receivers(RecArgs A) {
             const int gr = A.ibool[size_t(ce) * NP + iz * NG + l];
             const int gc = A.ibool[size_t(ce) * NP + l * NG + ix];
             const float hx = A.quad.hp[ix * NG + l], hz = A.quad.hp[iz * NG + l];
-            dxi0 += hx * A.u[size_t(gr) * nc];
-            dxi1 += hx * A.u[size_t(gr) * nc + 1];
-            dga0 += hz * A.u[size_t(gc) * nc];
-            dga1 += hz * A.u[size_t(gc) * nc + 1];
+            dxi0 += hx * ld_dep(A.u + size_t(gr) * nc);
+            dxi1 += hx * ld_dep(A.u + size_t(gr) * nc + 1);
+            dga0 += hz * ld_dep(A.u + size_t(gc) * nc);
+            dga1 += hz * ld_dep(A.u + size_t(gc) * nc + 1);
           }
           if (on && ty == 3 && nc == 4) {
             // pore pressure -(C div u_s + M div w) (poroelastic/isotropic/wavefield.hpp)
@@ -1014,10 +1133,10 @@ __global__ void __launch_bounds__(32) k_receivers(RecArgs A) {
               const int gr = A.ibool[size_t(ce) * NP + iz * NG + l];
               const int gc = A.ibool[size_t(ce) * NP + l * NG + ix];
               const float hx = A.quad.hp[ix * NG + l], hz = A.quad.hp[iz * NG + l];
-              dxi2 += hx * A.u[size_t(gr) * 4 + 2];
-              dxi3 += hx * A.u[size_t(gr) * 4 + 3];
-              dga2 += hz * A.u[size_t(gc) * 4 + 2];
-              dga3 += hz * A.u[size_t(gc) * 4 + 3];
+              dxi2 += hx * ld_dep(A.u + size_t(gr) * 4 + 2);
+              dxi3 += hx * ld_dep(A.u + size_t(gr) * 4 + 3);
+              dga2 += hz * ld_dep(A.u + size_t(gc) * 4 + 2);
+              dga3 += hz * ld_dep(A.u + size_t(gc) * 4 + 3);
             }
             const float dux = A.xix[p] * dxi0 + A.gax[p] * dga0;
             const float duz = A.xiz[p] * dxi1 + A.gaz[p] * dga1;
@@ -1034,20 +1153,20 @@ __global__ void __launch_bounds__(32) k_receivers(RecArgs A) {
             const float duxz = A.xiz[p] * dxi0 + A.gaz[p] * dga0;
             const float duzx = A.xix[p] * dxi1 + A.gax[p] * dga1;
             const float curl = duxz - duzx;
-            pr = ty == 6 ? curl : A.u[size_t(g) * 3 + 2] - 0.5f * curl;
+            pr = ty == 6 ? curl : ld_dep(A.u + size_t(g) * 3 + 2) - 0.5f * curl;
           }
         }
         o[0] = warp_sum(h * pr);
       } else if (ty == 4) {                    // Cosserat rotation
-        o[0] = warp_sum(nc == 3 ? h * A.u[size_t(g) * 3 + 2] : 0.f);
+        o[0] = warp_sum(nc == 3 ? h * ld_dep(A.u + size_t(g) * 3 + 2) : 0.f);
       } else {
         for (int c = 0; c < (nc < 2 ? nc : 2); ++c) {
           const size_t k = size_t(g) * A.ncomp + c;
           float val = 0.f;
           switch (A.types[t]) {
-            case 0: val = A.u[k]; break;
-            case 1: val = A.final_fields ? A.v[k] : newmark_correct(A.v[k], rec_accel(A, g, c), A.dt2); break;
-            default: val = A.final_fields ? A.a[k] : rec_accel(A, g, c); break;
+            case 0: val = ld_dep(A.u + k); break;
+            case 1: if (!EARLY) val = A.final_fields ? A.v[k] : newmark_correct(ld_dep(A.v + k), rec_accel(A, g, c), A.dt2); break;
+            default: if (!EARLY) val = A.final_fields ? A.a[k] : rec_accel(A, g, c); break;
           }
           o[c] = warp_sum(h * val);
         }
@@ -1061,10 +1180,10 @@ __global__ void __launch_bounds__(32) k_receivers(RecArgs A) {
     return;
   }
   // acoustic: displacement-like outputs are rho^-1 grad(field); pressure = -chi_dd
-  const float a = A.final_fields ? A.a[g] : rec_accel(A, g, 0);
+  const float a = EARLY ? 0.f : (A.final_fields ? A.a[g] : rec_accel(A, g, 0));
   if (on) {
-    sf[0][q] = A.u[g];
-    sf[1][q] = A.final_fields ? A.v[g] : newmark_correct(A.v[g], a, A.dt2);
+    sf[0][q] = ld_dep(A.u + g);
+    sf[1][q] = EARLY ? 0.f : (A.final_fields ? A.v[g] : newmark_correct(ld_dep(A.v + g), a, A.dt2));
     sf[2][q] = a;
   }
   __syncwarp();
@@ -1096,6 +1215,13 @@ __global__ void __launch_bounds__(32) k_receivers(RecArgs A) {
       dst[1] = oz;
     }
   }
+}
+
+__global__ void __launch_bounds__(32) k_receivers(const __grid_constant__ RecArgs A) {
+  __shared__ float sf[3 * NP];
+  pdl_wait();
+  pdl_release();
+  receiver_warp<false>(A, blockIdx.x, threadIdx.x, sf);
 }
 
 }  // namespace dev

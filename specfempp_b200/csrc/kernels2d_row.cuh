@@ -48,11 +48,12 @@ __device__ __forceinline__ void elastic_rows(const StiffArgs &S, const MedArgs &
     ggax[ix] = __ldg(A.gax + pe + ix); ggaz[ix] = __ldg(A.gaz + pe + ix);
     gjac[ix] = __ldg(A.jac + pe + ix); gc0[ix] = __ldg(A.prop0 + pe + ix); gmu[ix] = __ldg(A.prop1 + pe + ix);
   }
+  pdl_wait();
+  pdl_release();
 #pragma unroll
-  for (int ix = 0; ix < NG; ++ix) {
-    ur[ix] = act ? reinterpret_cast<const float2 *>(A.u)[g[ix]] : make_float2(0.f, 0.f);
-    su[iz * NG + ix] = ur[ix];
-  }
+  for (int ix = 0; ix < NG; ++ix) ur[ix] = act ? ld_dep2(A.u + size_t(g[ix]) * 2) : make_float2(0.f, 0.f);
+#pragma unroll
+  for (int ix = 0; ix < NG; ++ix) su[iz * NG + ix] = ur[ix];
   float hz[NG];
 #pragma unroll
   for (int l = 0; l < NG; ++l) hz[l] = c_hp[iz * NG + l];
@@ -113,7 +114,7 @@ __device__ __forceinline__ void elastic_rows(const StiffArgs &S, const MedArgs &
       const float wq = A.bc_w[k];
       if (wq != 0.f) {
         const float nx = A.bc_nx[k], nz = A.bc_nz[k], j1 = A.bc_j1[k];
-        const float2 vv = reinterpret_cast<const float2 *>(A.v)[g[ix]];
+        const float2 vv = ld_dep2(A.v + size_t(g[ix]) * 2);
         const float rvp = A.bc_imp0[k], rvs = A.bc_imp1[k];
         const float vn = vv.x * nx + vv.y * nz;
         const float fx = ((vn * nx / (j1 * j1)) * (rvp - rvs)) + vv.x * rvs;
@@ -123,9 +124,9 @@ __device__ __forceinline__ void elastic_rows(const StiffArgs &S, const MedArgs &
       }
     }
     if (src >= 0) {
-      const int step = *S.step;
+      const int step = ld_dep(S.step);
       for (int s = src; s >= 0; s = S.src_next[s]) {
-        const float f = step < S.nstep ? S.stf[size_t(step) * S.nsrc + s] : 0.f;
+        const float f = step < S.nstep ? ld_dep(S.stf + size_t(step) * S.nsrc + s) : 0.f;
         a0 += f * S.src_arr[(size_t(s) * 2 + 0) * NP + q];
         a1 += f * S.src_arr[(size_t(s) * 2 + 1) * NP + q];
       }
@@ -157,11 +158,12 @@ __device__ __forceinline__ void acoustic_rows(const StiffArgs &S, const MedArgs 
     ggax[ix] = __ldg(A.gax + pe + ix); ggaz[ix] = __ldg(A.gaz + pe + ix);
     gjac[ix] = __ldg(A.jac + pe + ix); grho[ix] = __ldg(A.prop0 + pe + ix);
   }
+  pdl_wait();
+  pdl_release();
 #pragma unroll
-  for (int ix = 0; ix < NG; ++ix) {
-    ur[ix] = act ? A.u[g[ix]] : 0.f;
-    su[iz * NG + ix] = ur[ix];
-  }
+  for (int ix = 0; ix < NG; ++ix) ur[ix] = act ? ld_dep(A.u + g[ix]) : 0.f;
+#pragma unroll
+  for (int ix = 0; ix < NG; ++ix) su[iz * NG + ix] = ur[ix];
   float hz[NG];
 #pragma unroll
   for (int l = 0; l < NG; ++l) hz[l] = c_hp[iz * NG + l];
@@ -200,13 +202,13 @@ __device__ __forceinline__ void acoustic_rows(const StiffArgs &S, const MedArgs 
     if (bs >= 0) {
       const size_t k = size_t(bs) * NP + q;
       const float wq = A.bc_w[k];
-      if (wq != 0.f) a += -1.f * (wq * A.bc_j1[k]) * A.bc_imp0[k] * A.v[g[ix]];
+      if (wq != 0.f) a += -1.f * (wq * A.bc_j1[k]) * A.bc_imp0[k] * ld_dep(A.v + g[ix]);
       a *= A.bc_keep[k];   // acoustic free surface (Dirichlet) zeroes the element term
     }
     if (src >= 0) {
-      const int step = *S.step;
+      const int step = ld_dep(S.step);
       for (int s = src; s >= 0; s = S.src_next[s]) {
-        const float f = step < S.nstep ? S.stf[size_t(step) * S.nsrc + s] : 0.f;
+        const float f = step < S.nstep ? ld_dep(S.stf + size_t(step) * S.nsrc + s) : 0.f;
         a += f * S.src_arr[(size_t(s) * 2) * NP + q];
       }
     }
@@ -214,14 +216,17 @@ __device__ __forceinline__ void acoustic_rows(const StiffArgs &S, const MedArgs 
   }
 }
 
-// Blocks [0, el.nblocks) run elastic P-SV elements, the others acoustic ones.
+// The first rec_blocks blocks take receivers, the next el.nblocks elastic P-SV elements, the others acoustic ones.
 template <int E>
 __global__ void __launch_bounds__(NG * E, E == 16 ? 8 : (E == 32 ? 4 : 1)) k_stiffness_row(StiffArgs S) {
   __shared__ __align__(16) float2 smem[2 * E * NP];
-  if (int(blockIdx.x) < S.el.nblocks)
-    elastic_rows<E>(S, S.el, S.el.e0 + blockIdx.x * E, smem);
+  const int b = int(blockIdx.x) - S.rec_blocks;
+  if (b < 0)
+    receiver_blocks(S.rec_ac, S.rec_el, S.nrec_ac, S.nrec_el, reinterpret_cast<float *>(smem));
+  else if (b < S.el.nblocks)
+    elastic_rows<E>(S, S.el, S.el.e0 + b * E, smem);
   else
-    acoustic_rows<E>(S, S.ac, S.ac.e0 + (blockIdx.x - S.el.nblocks) * E, reinterpret_cast<float *>(smem));
+    acoustic_rows<E>(S, S.ac, S.ac.e0 + (b - S.el.nblocks) * E, reinterpret_cast<float *>(smem));
 }
 
 }  // namespace dev

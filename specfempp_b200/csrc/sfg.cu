@@ -206,6 +206,11 @@ struct sfg_handle {
   int *d_src_next = nullptr, *d_src_shot = nullptr;
   float *d_src_arr = nullptr, *d_stf = nullptr;
   float *d_src_arr2 = nullptr;     // poroelastic fluid rows of the source arrays
+  // receiver arguments (acoustic, elastic) on the device, read by the element
+  // launches that take the early receivers; early_now: the media whose early
+  // receivers the next element launch takes (set around it by enqueue_step)
+  sfg::dev::RecArgs *d_rec_args = nullptr;
+  bool early_now[2] = {false, false};
   int *d_rec_elem = nullptr;
   float *d_rec_h = nullptr, *d_seis = nullptr;
   int *d_step = nullptr, *d_flag = nullptr;
@@ -385,6 +390,39 @@ sfg::dev::MedArgs med_args(const DevMedium &D) {
 
 int ncolors(const DevMedium &D) { return D.nspec ? int(D.color_start.size()) - 1 : 0; }
 
+// Launch as a programmatic dependent of the kernel before it on the stream
+// (pdl_wait in kernels2d.cuh): only for kernels that call pdl_wait on every
+// thread before they touch data of the step.
+template <typename... P, typename... A>
+void launch_pdl(void (*kern)(P...), int grid, int block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(unsigned(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  SFG_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
+}
+
+// Whether the step is the single-shot owner-computes chain (element kernel,
+// late receivers, point update) whose kernels are launched as programmatic
+// dependents and whose early receivers ride in the element launch.
+bool chained(const sfg_handle *h) { return h->asmb.nshots == 1 && (h->variant == 3 || h->variant == 6); }
+
+// The early receivers of a launch, one warp each, in its first blocks.
+void early_receivers(const sfg_handle *h, sfg::dev::StiffArgs &S, int threads, bool ac, bool el) {
+  S.nrec_ac = ac ? h->ac.nrec : 0;
+  S.nrec_el = el ? h->el.nrec : 0;
+  S.rec_ac = h->d_rec_args;
+  S.rec_el = h->d_rec_args + 1;
+  const int nw = threads / 32;
+  S.rec_blocks = (S.nrec_ac + S.nrec_el + nw - 1) / nw;
+}
+
 template <int E, int EK>
 void launch_stiffness_E(sfg_handle *h, const DevMedium &el, const DevMedium &ac, const int *step,
                         cudaStream_t s, int variant) {
@@ -410,8 +448,9 @@ void launch_stiffness_E(sfg_handle *h, const DevMedium &el, const DevMedium &ac,
     // owner-computes: one launch over every element of both media
     S.el.e0 = 0; S.el.e1 = el.nspec; S.el.nblocks = (el.nspec + E - 1) / E;
     S.ac.e0 = 0; S.ac.e1 = ac.nspec; S.ac.nblocks = (ac.nspec + E - 1) / E;
-    const int grid = S.el.nblocks + S.ac.nblocks;
-    if (grid > 0) sfg::dev::k_stiffness<E, EK, true><<<grid, sfg::dev::NP * E, 0, s>>>(S);
+    early_receivers(h, S, sfg::dev::NP * E, h->early_now[0], h->early_now[1]);
+    const int grid = S.el.nblocks + S.ac.nblocks + S.rec_blocks;
+    if (grid > 0) launch_pdl(sfg::dev::k_stiffness<E, EK, true>, grid, sfg::dev::NP * E, 0, s, S);
     return;
   }
   if (variant == 4) {
@@ -587,8 +626,9 @@ void launch_stiffness_row(sfg_handle *h, const DevMedium &el, const DevMedium &a
   S.quad = h->quad;
   S.el.e0 = 0; S.el.e1 = el.nspec; S.el.nblocks = (el.nspec + E - 1) / E;
   S.ac.e0 = 0; S.ac.e1 = ac.nspec; S.ac.nblocks = (ac.nspec + E - 1) / E;
-  const int grid = S.el.nblocks + S.ac.nblocks;
-  if (grid > 0) sfg::dev::k_stiffness_row<E><<<grid, sfg::dev::NG * E, 0, s>>>(S);
+  early_receivers(h, S, sfg::dev::NG * E, h->early_now[0], h->early_now[1]);
+  const int grid = S.el.nblocks + S.ac.nblocks + S.rec_blocks;
+  if (grid > 0) launch_pdl(sfg::dev::k_stiffness_row<E>, grid, sfg::dev::NG * E, 0, s, S);
 }
 
 void launch_stiffness(sfg_handle *h, const DevMedium &el, const DevMedium &ac, const int *step,
@@ -736,6 +776,7 @@ void launch_receivers(sfg_handle *h, int medium, cudaStream_t s) {
   if (D.nrec == 0) return;
   const sfg::dev::RecArgs R = rec_args(h, medium);
   if (D.S > 1) sfg::dev::k_receivers_batched<<<D.nrec, 32, 0, s>>>(R, D.S);
+  else if (chained(h)) launch_pdl(sfg::dev::k_receivers, D.nrec, 32, 0, s, R);
   else sfg::dev::k_receivers<<<D.nrec, 32, 0, s>>>(R);
 }
 
@@ -743,13 +784,19 @@ void launch_update(sfg_handle *h, int medium, bool predict, bool advance, cudaSt
   const DevMedium &D = medium == SFG_MEDIUM_ELASTIC ? h->el : h->ac;
   const DevMedium &O = medium == SFG_MEDIUM_ELASTIC ? h->ac : h->el;
   sfg::dev::UpdateArgs U = update_args(h, D, O, medium, predict, advance);
+  if (chained(h)) {
+    const int grid = grid_for(U.n / D.ncomp);
+    if (D.ncomp == 2) launch_pdl(sfg::dev::k_update_gather<2>, grid, 256, 0, s, U);
+    else if (D.ncomp == 3) launch_pdl(sfg::dev::k_update_gather<3>, grid, 256, 0, s, U);
+    else if (D.ncomp == 4) launch_pdl(sfg::dev::k_update_gather<4>, grid, 256, 0, s, U);
+    else launch_pdl(sfg::dev::k_update_gather<1>, grid, 256, 0, s, U);
+    return;
+  }
   if (h->variant >= 3) {
     if (D.S > 1 && D.S % 4 == 0)
       sfg::dev::k_update_batched4_gather<<<grid_for(U.n / 4), 256, 0, s>>>(U, D.S, D.ncomp);
     else if (D.S > 1) sfg::dev::k_update_batched_gather<<<grid_for(U.n), 256, 0, s>>>(U, D.S, D.ncomp);
     else if (D.ncomp == 2) sfg::dev::k_update_gather<2><<<grid_for(U.n / 2), 256, 0, s>>>(U);
-    else if (D.ncomp == 3) sfg::dev::k_update_gather<3><<<grid_for(U.n / 3), 256, 0, s>>>(U);
-    else if (D.ncomp == 4) sfg::dev::k_update_gather<4><<<grid_for(U.n / 4), 256, 0, s>>>(U);
     else sfg::dev::k_update_gather<1><<<grid_for(U.n), 256, 0, s>>>(U);
     return;
   }
@@ -764,7 +811,8 @@ void launch_update_coupled(sfg_handle *h, bool predict, cudaStream_t s) {
   sfg::dev::UpdateArgs E = update_args(h, h->el, h->ac, SFG_MEDIUM_ELASTIC, predict, true);
   sfg::dev::UpdateArgs A = update_args(h, h->ac, h->el, SFG_MEDIUM_ACOUSTIC, predict, false);
   const int n = E.n / 2 + A.n - A.niface;
-  sfg::dev::k_update_coupled<<<grid_for(n), 256, 0, s>>>(E, A);
+  if (chained(h)) launch_pdl(sfg::dev::k_update_coupled, grid_for(n), 256, 0, s, E, A);
+  else sfg::dev::k_update_coupled<<<grid_for(n), 256, 0, s>>>(E, A);
 }
 
 // Whether this step may use launch_update_coupled: owner-computes, one shot,
@@ -1287,6 +1335,24 @@ void enqueue_step(sfg_handle *h, cudaStream_t s, bool predict) {
   const bool rec_el = has_el && h->el.nrec > 0 && h->recording != 2;
   const bool early_ac = rec_ac && receivers_early(h, SFG_MEDIUM_ACOUSTIC);
   const bool early_el = rec_el && receivers_early(h, SFG_MEDIUM_ELASTIC);
+  if (chained(h)) {
+    // the early receivers ride in the element launch
+    h->early_now[0] = early_ac;
+    h->early_now[1] = early_el;
+    launch_stiffness(h, s);
+    h->early_now[0] = h->early_now[1] = false;
+    const bool both = fused_update(h);
+    if (rec_ac && !early_ac) launch_receivers(h, SFG_MEDIUM_ACOUSTIC, s);
+    if (both) {
+      if (rec_el && !early_el) launch_receivers(h, SFG_MEDIUM_ELASTIC, s);
+      launch_update_coupled(h, predict, s);
+      return;
+    }
+    if (has_ac) launch_update(h, SFG_MEDIUM_ACOUSTIC, predict, !has_el, s);
+    if (rec_el && !early_el) launch_receivers(h, SFG_MEDIUM_ELASTIC, s);
+    if (has_el) launch_update(h, SFG_MEDIUM_ELASTIC, predict, true, s);
+    return;
+  }
   const bool fork = (early_ac || early_el) && h->side;
   if (fork) {
     // receivers on the side stream, concurrent with the element kernel; they
@@ -1319,9 +1385,10 @@ int kernels_per_step(const sfg_handle *h) {
   if (h->variant == 5) return 2 + (h->el.nspec && h->el.nrec > 0) + (h->ac.nspec && h->ac.nrec > 0);
   if (h->variant == 7) return 2 + (h->el.nrec > 0);
   int n = h->variant >= 3 ? 1 : std::max(ncolors(h->el), ncolors(h->ac));
-  for (const DevMedium *D : {&h->ac, &h->el}) {
-    if (D->nspec == 0) continue;
-    n += (D->nrec > 0 ? 1 : 0) + 1;
+  for (int med : {SFG_MEDIUM_ACOUSTIC, SFG_MEDIUM_ELASTIC}) {
+    const DevMedium &D = med == SFG_MEDIUM_ELASTIC ? h->el : h->ac;
+    if (D.nspec == 0) continue;
+    n += (D.nrec > 0 && !(chained(h) && receivers_early(h, med)) ? 1 : 0) + 1;
   }
   return fused_update(h) ? n - 1 : n;
 }
@@ -1744,6 +1811,8 @@ int sfg_initialize(sfg_handle *h) {
     h->d_seis = h->mem.zeros<float>(size_t(a.nshots) * a.nsig * a.ntypes * std::max(a.nrec, 1) * 2);
     h->d_step = h->mem.zeros<int>(1);
     h->d_flag = h->mem.zeros<int>(1);
+    h->d_rec_args = h->mem.upload(std::vector<sfg::dev::RecArgs>{rec_args(h, SFG_MEDIUM_ACOUSTIC),
+                                                                  rec_args(h, SFG_MEDIUM_ELASTIC)});
     SFG_CUDA(cudaDeviceSynchronize());
     {
       int dev = 0;
