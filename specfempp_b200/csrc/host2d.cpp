@@ -507,6 +507,8 @@ bool read_database2d(const std::string &path, Mesh2D &m, std::string &err) {
 // --------------------------------------------------- model-dependent part ---
 // Material words, Stacey impedances, the assembled Stacey matrices and the
 // inverse mass matrix: everything that changes when the model changes.
+void classify_rows(MediumData &D);
+
 void assemble_model2d(const Mesh2D &m, Assembly2D &a) {
   const double dt = a.dt;
   double w[NGLL];
@@ -724,6 +726,33 @@ void assemble_model2d(const Mesh2D &m, Assembly2D &a) {
     D.minv.resize(M.size());
     for (size_t i = 0; i < M.size(); ++i) D.minv[i] = float(1.0 / M[i]);
   }
+  classify_rows(a.el);
+  classify_rows(a.ac);
+}
+
+// What the row-form element kernel may read once an element (RowClass).
+void classify_rows(MediumData &D) {
+  MediumData::RowClass &R = D.row;
+  const int rw = D.poro ? 16 : 8;
+  R.erec.assign(size_t(D.nspec) * rw, 0.0f);
+  bool straight = true, matconst = true;
+#pragma omp parallel for schedule(static) reduction(&& : straight, matconst)
+  for (int ce = 0; ce < D.nspec; ++ce) {
+    const size_t p = size_t(ce) * NPTS;
+    for (size_t k = p; k < p + NPTS; ++k) {
+      straight = straight && D.xiz[k] == 0.0f && D.gax[k] == 0.0f && D.xix[k] == D.xix[p] &&
+                 D.gaz[k] == D.gaz[p] && D.jac[k] == D.jac[p];
+      matconst = matconst && D.prop0[k] == D.prop0[p] && D.prop1[k] == D.prop1[p];
+    }
+    float *r = &R.erec[size_t(ce) * rw];
+    r[0] = D.xix[p]; r[1] = D.gaz[p]; r[2] = D.jac[p]; r[4] = D.prop0[p]; r[5] = D.prop1[p];
+    if (D.poro) {          // material constants only: one value an element
+      r[8] = D.prop2[p]; r[9] = D.prop3[p]; r[10] = D.prop4[p]; r[11] = D.prop5[p];
+      r[12] = D.prop6[p]; r[13] = D.prop7[p]; r[14] = D.prop8[p];
+    }
+  }
+  R.straight = straight;
+  R.matconst = matconst;
 }
 
 void set_model2d(Mesh2D &m, Assembly2D &a, const float *rho, const float *kappa, const float *mu) {
@@ -821,6 +850,25 @@ void assemble2d(const Mesh2D &m, double dt, Assembly2D &a) {
         a.gx[p] = J[p].x;
         a.gz[p] = J[p].z;
       }
+  // An element that is a rectangle along the axes up to the rounding of its
+  // control nodes (1e-10 of its derivatives, far below the FP32 words that
+  // the kernels read) gets exactly that geometry: zero cross derivatives and
+  // one value of the others.
+  for (int e = 0; e < nspec; ++e) {
+    JacD *E = &J[size_t(e) * NPTS];
+    const JacD C = E[NPTS / 2];
+    const double xxi = C.gaz * C.jac, zga = C.xix * C.jac, tol = 1e-10;
+    bool rect = true;
+    for (int q = 0; q < NPTS && rect; ++q)
+      rect = std::abs(E[q].xiz * E[q].jac) <= tol * xxi && std::abs(E[q].gax * E[q].jac) <= tol * zga &&
+             std::abs(E[q].gaz * E[q].jac - xxi) <= tol * xxi && std::abs(E[q].xix * E[q].jac - zga) <= tol * zga;
+    if (!rect) continue;
+    for (int q = 0; q < NPTS; ++q) {
+      E[q].xix = 1.0 / xxi; E[q].gaz = 1.0 / zga;
+      E[q].xiz = E[q].gax = 0.0;
+      E[q].jac = xxi * zga;
+    }
+  }
 
   // --- media and colouring ------------------------------------------
   a.mesh_medium.resize(nspec);

@@ -76,6 +76,15 @@ struct MediumData {
   // inverse permeability (xx, xz, zz)
   bool poro = false;
   std::vector<float> prop6, prop7, prop8;
+  // Row-form element kernel: what is one value an element.  straight: every
+  // element is a rectangle along the axes (xi_z and gamma_x zero, xi_x,
+  // gamma_z and |J| constant, bit for bit); matconst: so are the material
+  // words.  erec [nspec][8]: xi_x, gamma_z, |J|, 0, prop0, prop1, 0, 0 of the
+  // element's first point; poroelastic [nspec][16]: then prop2..prop8, 0.
+  struct RowClass {
+    bool straight = false, matconst = false;
+    std::vector<float> erec;
+  } row;
   std::vector<float> minv;            // [nglob][ncomp]
   // Stacey / free-surface: slot per element (-1 none), compact [nslot][25]
   std::vector<int> bc_slot;

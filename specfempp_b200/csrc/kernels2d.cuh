@@ -100,6 +100,7 @@ struct MedArgs {
       *__restrict__ jac, *__restrict__ prop0, *__restrict__ prop1;
   const float *__restrict__ prop2, *__restrict__ prop3, *__restrict__ prop4, *__restrict__ prop5;  // anisotropic
   const float *__restrict__ prop6, *__restrict__ prop7, *__restrict__ prop8;  // poroelastic damping
+  const float *__restrict__ erec;   // row form: per-element records (RowClass)
   const int *__restrict__ bc_slot;
   const float *__restrict__ bc_w, *__restrict__ bc_nx, *__restrict__ bc_nz, *__restrict__ bc_j1,
       *__restrict__ bc_imp0, *__restrict__ bc_imp1, *__restrict__ bc_keep;

@@ -196,8 +196,7 @@ __global__ void __launch_bounds__(NG * E, 4) k_adj_elem_row(AdjArgs A) {
     gjac[ix] = __ldg(A.jac + pe + ix); gc0[ix] = __ldg(A.prop0 + pe + ix); gmu[ix] = __ldg(A.prop1 + pe + ix);
   }
   float hz[NG];
-#pragma unroll
-  for (int l = 0; l < NG; ++l) hz[l] = c_hp[iz * NG + l];
+  ld_row5(t_rows[iz], hz);
   __syncthreads();
   // xi derivatives of both fields, both components paired, in place
   {
@@ -216,7 +215,7 @@ __global__ void __launch_bounds__(NG * E, 4) k_adj_elem_row(AdjArgs A) {
 #pragma unroll
     for (int ix = 0; ix < NG; ++ix) { mr[ix] = dm[ix]; ur[ix] = du[ix]; }
   }
-  const float wiz = c_w[iz];
+  const float wiz = ld_w(iz);
 #pragma unroll
   for (int ix = 0; ix < NG; ++ix) {
     const size_t p = pe + ix;
@@ -253,8 +252,7 @@ __global__ void __launch_bounds__(NG * E, 4) k_adj_elem_row(AdjArgs A) {
     }
   }
   float wz[NG];
-#pragma unroll
-  for (int l = 0; l < NG; ++l) wz[l] = c_hpw[l * NG + iz];
+  ld_row5(t_rows[5 + iz], wz);
   __syncthreads();
   if (!act) return;
 #pragma unroll

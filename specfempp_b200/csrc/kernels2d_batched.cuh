@@ -26,6 +26,26 @@ __constant__ float c_hp[NP];    // hp[i*5+j] = l'_j(xi_i)
 __constant__ float c_hpw[NP];   // hp[l*5+i] * w[l]
 __constant__ float c_w[NG];
 
+// The same coefficients in global memory, for threads of a warp that need
+// different rows: indexed constant-bank loads are served one address at a
+// time (the indexed-constant unit was 77% busy in the acoustic row kernel,
+// whose compiler reloads them at every use), a row here is two L1 hits and
+// stays in registers.  Row i: l'_l(xi_i) over l; row 5 + i: hpw[l*5+i] over l;
+// [10][i]: w.
+__device__ __align__(16) float t_rows[11][8];
+
+__device__ __forceinline__ void ld_row5(const float *row, float (&h)[NG]) {
+  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(h[0]), "=f"(h[1]), "=f"(h[2]), "=f"(h[3])
+               : "l"(row));
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(h[4]) : "l"(row + 4));
+}
+__device__ __forceinline__ float ld_w(int i) {
+  float x;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(x) : "l"(&t_rows[10][i]));
+  return x;
+}
+
 struct BatchArgs {
   const int *__restrict__ ibool;
   const float *__restrict__ xix, *__restrict__ xiz, *__restrict__ gax, *__restrict__ gaz,

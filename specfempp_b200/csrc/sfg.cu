@@ -82,6 +82,7 @@ struct DevMedium {
         *prop0 = nullptr, *prop1 = nullptr;
   float *prop2 = nullptr, *prop3 = nullptr, *prop4 = nullptr, *prop5 = nullptr;  // anisotropic / Cosserat
   float *prop6 = nullptr, *prop7 = nullptr, *prop8 = nullptr;                      // poroelastic damping
+  float *erec = nullptr;                                                           // row form: element records
   bool aniso = false, poro = false;
   int *bc_slot = nullptr;
   float *bc_w = nullptr, *bc_nx = nullptr, *bc_nz = nullptr, *bc_j1 = nullptr,
@@ -343,6 +344,7 @@ void upload_medium(sfg_handle *h, const sfg::MediumData &M, DevMedium &D) {
     D.prop5 = padded(M.prop5); D.prop6 = padded(M.prop6); D.prop7 = padded(M.prop7);
     D.prop8 = padded(M.prop8);
   }
+  D.erec = m.upload(M.row.erec);
   D.bc_slot = m.upload(M.bc_slot);
   D.bc_w = m.upload(M.bc_w); D.bc_nx = m.upload(M.bc_nx); D.bc_nz = m.upload(M.bc_nz);
   D.bc_j1 = m.upload(M.bc_j1); D.bc_imp0 = m.upload(M.bc_imp0); D.bc_imp1 = m.upload(M.bc_imp1);
@@ -380,6 +382,7 @@ sfg::dev::MedArgs med_args(const DevMedium &D) {
   A.prop0 = D.prop0; A.prop1 = D.prop1;
   A.prop2 = D.prop2; A.prop3 = D.prop3; A.prop4 = D.prop4; A.prop5 = D.prop5;
   A.prop6 = D.prop6; A.prop7 = D.prop7; A.prop8 = D.prop8;
+  A.erec = D.erec;
   A.bc_slot = D.bc_slot; A.bc_w = D.bc_w; A.bc_nx = D.bc_nx; A.bc_nz = D.bc_nz;
   A.bc_j1 = D.bc_j1; A.bc_imp0 = D.bc_imp0; A.bc_imp1 = D.bc_imp1; A.bc_keep = D.bc_keep;
   A.bc_imp2 = D.bc_imp2;
@@ -607,8 +610,22 @@ void launch_stiffness_batched(sfg_handle *h, const DevMedium &el, const int *ste
   }
 }
 
-// The row-form kernel covers isotropic P-SV and acoustic media.
-bool row_ok(const DevMedium &el) { return el.nspec == 0 || (el.ncomp == 2 && !el.aniso); }
+// The row-form kernel covers isotropic P-SV and acoustic media, and SH and
+// poroelastic media alone.
+bool row_ok(const DevMedium &el, const DevMedium &ac) {
+  if (el.nspec == 0 || (el.ncomp == 2 && !el.aniso)) return true;
+  return ac.nspec == 0 && (el.ncomp == 1 || el.ncomp == 4);
+}
+
+// The element kernel's specialisation: what is one value an element in every
+// medium of the model (RowClass).  Unlike the geometry, the material can
+// change (sfg_set_model2d, which captures the step graphs again).
+bool row_straight(const sfg_handle *h) {
+  return (!h->el.nspec || h->asmb.el.row.straight) && (!h->ac.nspec || h->asmb.ac.row.straight);
+}
+bool row_matconst(const sfg_handle *h) {
+  return (!h->el.nspec || h->asmb.el.row.matconst) && (!h->ac.nspec || h->asmb.ac.row.matconst);
+}
 
 template <int E>
 void launch_stiffness_row(sfg_handle *h, const DevMedium &el, const DevMedium &ac, const int *step,
@@ -628,7 +645,25 @@ void launch_stiffness_row(sfg_handle *h, const DevMedium &el, const DevMedium &a
   S.ac.e0 = 0; S.ac.e1 = ac.nspec; S.ac.nblocks = (ac.nspec + E - 1) / E;
   early_receivers(h, S, sfg::dev::NG * E, h->early_now[0], h->early_now[1]);
   const int grid = S.el.nblocks + S.ac.nblocks + S.rec_blocks;
-  if (grid > 0) launch_pdl(sfg::dev::k_stiffness_row<E>, grid, sfg::dev::NG * E, 0, s, S);
+  if (grid == 0) return;
+  if (!S.el.erec && !S.ac.erec) throw std::runtime_error("row-form element kernel: element records missing on the device");
+  const int geo = row_straight(h) ? 1 : 0, mat = row_matconst(h) ? 1 : 0;
+  auto go = [&](auto kern) { launch_pdl(kern, grid, sfg::dev::NG * E, 0, s, S); };
+  if (el.nspec && el.ncomp == 4) {
+    if (geo) go(sfg::dev::k_stiffness_row<E, 4, 1, 1>);
+    else go(sfg::dev::k_stiffness_row<E, 4, 0, 1>);
+    return;
+  }
+  auto pick = [&](auto ek) {
+    constexpr int EK = decltype(ek)::value;
+    if (geo && mat) go(sfg::dev::k_stiffness_row<E, EK, 1, 1>);
+    else if (geo) go(sfg::dev::k_stiffness_row<E, EK, 1, 0>);
+    else if (mat) go(sfg::dev::k_stiffness_row<E, EK, 0, 1>);
+    else go(sfg::dev::k_stiffness_row<E, EK, 0, 0>);
+  };
+  if (el.nspec == 0) pick(std::integral_constant<int, 5>{});
+  else if (el.ncomp == 1) pick(std::integral_constant<int, 1>{});
+  else pick(std::integral_constant<int, 0>{});
 }
 
 void launch_stiffness(sfg_handle *h, const DevMedium &el, const DevMedium &ac, const int *step,
@@ -639,7 +674,7 @@ void launch_stiffness(sfg_handle *h, const DevMedium &el, const DevMedium &ac, c
   }
   if (variant == 6) {
     // owner-computes with the row-form element kernel (16 or 32 elements per block)
-    if (row_ok(el)) {
+    if (row_ok(el, ac)) {
       if (h->epb == 16) launch_stiffness_row<16>(h, el, ac, step, s);
       else launch_stiffness_row<32>(h, el, ac, step, s);
       return;
@@ -1413,6 +1448,18 @@ cudaGraphExec_t capture(sfg_handle *h, int nsteps, bool last_predicts) {
   return ex;
 }
 
+// Capture the step graphs (again); the streamed and the recording steps'
+// graphs are captured when they are next used.
+void recapture(sfg_handle *h) {
+  SFG_CUDA(cudaStreamSynchronize(h->stream));
+  for (cudaGraphExec_t *g : {&h->graph_k, &h->graph_1, &h->graph_e, &h->graph_io, &h->adj.graph_r1, &h->adj.graph_re,
+                             &h->adj.graph_rseg})
+    if (*g) { cudaGraphExecDestroy(*g); *g = nullptr; }
+  h->graph_k = capture(h, h->graph_steps, true);
+  h->graph_1 = capture(h, 1, true);
+  h->graph_e = capture(h, 1, false);
+}
+
 void resume(sfg_handle *h) {
   if (h->state_final) {
     launch_predict(h, h->stream);
@@ -1454,7 +1501,7 @@ void autotune(sfg_handle *h) {
   if (h->variant == 5 && !h->tile_ok) h->variant = 3;   // the model cannot use the tile kernel
   if (h->variant == 5) h->epb = 16;
   // the row form: isotropic P-SV / acoustic, one shot, 16 or 32 elements per block
-  if (h->variant == 6 && (h->asmb.nshots > 1 || !row_ok(h->el))) h->variant = 3;
+  if (h->variant == 6 && (h->asmb.nshots > 1 || !row_ok(h->el, h->ac))) h->variant = 3;
   if (h->variant == 6 && h->epb != 16) h->epb = 32;
   if (h->variant == 7 && !h->btile_ok) h->variant = 3;   // batched tiles of four elements
   if (h->asmb.nshots > 1 && h->variant == 2) h->variant = 1;  // no persistent batched kernel
@@ -1479,7 +1526,7 @@ void autotune(sfg_handle *h) {
     // fused tile kernel: tiles of 16 elements
     if (h->tile_ok && (!fix_v || h->variant == 5) && (!fix_e || h->epb == 16)) cand.push_back({5, 16});
     // row-form element kernel
-    if (row_ok(h->el) && (!fix_v || h->variant == 6))
+    if (row_ok(h->el, h->ac) && (!fix_v || h->variant == 6))
       for (int e : {16, 32})
         if (!fix_e || e == h->epb) cand.push_back({6, e});
   }
@@ -1797,6 +1844,17 @@ int sfg_initialize(sfg_handle *h) {
     SFG_CUDA(cudaMemcpyToSymbol(sfg::dev::c_hp, a.hprime, sizeof(a.hprime)));
     SFG_CUDA(cudaMemcpyToSymbol(sfg::dev::c_hpw, a.hpw, sizeof(a.hpw)));
     SFG_CUDA(cudaMemcpyToSymbol(sfg::dev::c_w, a.wgll, sizeof(a.wgll)));
+    {
+      float rows[11][8] = {};
+      for (int i = 0; i < sfg::NGLL; ++i) {
+        for (int l = 0; l < sfg::NGLL; ++l) {
+          rows[i][l] = a.hprime[i * sfg::NGLL + l];
+          rows[5 + i][l] = a.hpw[l * sfg::NGLL + i];
+        }
+        rows[10][i] = a.wgll[i];
+      }
+      SFG_CUDA(cudaMemcpyToSymbol(sfg::dev::t_rows, rows, sizeof(rows)));
+    }
     h->d_src_arr = h->mem.upload(a.src_arr);
     h->d_src_arr2 = a.src_arr2.empty() ? nullptr : h->mem.upload(a.src_arr2);
     h->d_stf = h->mem.upload(a.stf);
@@ -1836,9 +1894,7 @@ int sfg_initialize(sfg_handle *h) {
     if (h->btile_ok) upload_btiles(h);
     autotune(h);
     h->graph_steps = std::max(1, h->opt.steps_per_graph);
-    h->graph_k = capture(h, h->graph_steps, true);
-    h->graph_1 = capture(h, 1, true);
-    h->graph_e = capture(h, 1, false);
+    recapture(h);
     h->initialized = true;
     return int(SFG_OK);
   });
@@ -1957,10 +2013,12 @@ int sfg_step_io(sfg_handle *h, const float *stf_row, float *seis_row) {
     const int step = h->host_step;
     const int rowlen = a.ntypes * a.nrec * 2;
     const size_t io_bytes = 16 + 4 * size_t(a.nsrc) + 4 * size_t(a.nshots) * rowlen;
-    if (!h->graph_io) {
+    if (!h->io_host) {
       SFG_CUDA(cudaHostAlloc(&h->io_host, io_bytes, cudaHostAllocMapped));
       std::memset(h->io_host, 0, io_bytes);
       SFG_CUDA(cudaHostGetDevicePointer(&h->io_dev, h->io_host, 0));
+    }
+    if (!h->graph_io) {
       const int *io_d = static_cast<const int *>(h->io_dev);
       float *seis_d = reinterpret_cast<float *>(static_cast<char *>(h->io_dev) + 16 + 4 * size_t(a.nsrc));
       // one fused step (the next step's predictor applied in the update)
@@ -2314,6 +2372,7 @@ int sfg_compute_seismograms(sfg_handle *h, int isig) {
 int sfg_set_model2d(sfg_handle *h, const float *rho, const float *kappa, const float *mu) {
   return guarded(h, [&]() {
     if (!rho || !kappa || !mu) return int(SFG_ERR_ARG);
+    const bool mat0 = row_matconst(h);
     sfg::set_model2d(h->mesh, h->asmb, rho, kappa, mu);
     // pressure sources in acoustic elements carry l / kappa: rebuild them
     const bool ac_src = h->have_sources && h->asmb.ac.nspec > 0 && h->asmb.nsrc > 0;
@@ -2332,7 +2391,10 @@ int sfg_set_model2d(sfg_handle *h, const float *rho, const float *kappa, const f
         put(D.prop0, M.prop0); put(D.prop1, M.prop1);
         put(D.bc_imp0, M.bc_imp0); put(D.bc_imp1, M.bc_imp1);
         put(D.minv, M.minv);
+        put(D.erec, M.row.erec);
       }
+      // the step graphs hold the element kernel of the old model's class
+      if (row_matconst(h) != mat0 && h->variant == 6) recapture(h);
       refresh_tile_records(h);
       if (h->adj.st_c && !h->asmb.el.stacey_c.empty())
         SFG_CUDA(cudaMemcpy(h->adj.st_c, h->asmb.el.stacey_c.data(), h->asmb.el.stacey_c.size() * sizeof(float),
