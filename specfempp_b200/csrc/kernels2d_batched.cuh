@@ -62,6 +62,7 @@ struct BatchArgs {
   float *__restrict__ accum;
   float *__restrict__ r;               // owner-computes: [slot[element*25 + point]][NC][S]
   const int *__restrict__ slot;
+  const float *__restrict__ erec;      // per-element records (RowClass)
   int e0;                              // first element of the colour
   int S;                               // shots
   int nspec_b;                         // elements (persistent kernel)
@@ -173,28 +174,76 @@ __global__ void __launch_bounds__(NP * 32) k_stiffness_batched(BatchArgs A) {
   }
 }
 
-// Owner-computes update for [point][NC][S] fields: each (point, comp, shot)
-// gathers its element contributions in colour order (bitwise the colour
-// passes' sum), then M^-1, corrector and optional predictor.
-__global__ void __launch_bounds__(256) k_update_batched_gather(UpdateArgs A, int S, int NC) {
+// Owner-computes update for [point][NC][S] fields: a thread takes V shots (as
+// one vector; V divides S) of both components of a point, so that all its
+// field loads are in flight together and the contribution range is read once;
+// the contributions are summed in colour order (bitwise the colour passes'
+// sum), then M^-1, corrector and optional predictor.  One component and one
+// vector a thread, with three divisions for its index, reached 0.61 of the
+// DRAM's cycles.
+template <int V> struct ShotVec { float x[V]; };
+template <int V>
+__device__ __forceinline__ ShotVec<V> ld_shots(const float *p) {
+  ShotVec<V> r;
+  if constexpr (V == 4) {
+    const float4 t = *reinterpret_cast<const float4 *>(p);
+    r.x[0] = t.x; r.x[1] = t.y; r.x[2] = t.z; r.x[3] = t.w;
+  } else if constexpr (V == 2) {
+    const float2 t = *reinterpret_cast<const float2 *>(p);
+    r.x[0] = t.x; r.x[1] = t.y;
+  } else {
+    r.x[0] = *p;
+  }
+  return r;
+}
+template <int V>
+__device__ __forceinline__ void st_shots(float *p, const ShotVec<V> &r) {
+  if constexpr (V == 4) *reinterpret_cast<float4 *>(p) = make_float4(r.x[0], r.x[1], r.x[2], r.x[3]);
+  else if constexpr (V == 2) *reinterpret_cast<float2 *>(p) = make_float2(r.x[0], r.x[1]);
+  else *p = r.x[0];
+}
+
+template <int NC, int V>
+__global__ void __launch_bounds__(256) k_update_batched_gather(UpdateArgs A, int S) {
+  const int SV = S / V, n = A.n / (NC * V);
   const int stride = gridDim.x * blockDim.x;
   bool bad = false;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += stride) {
-    const int s = i % S;
-    const int gc = i / S;
-    const int g = gc / NC, c = gc - g * NC;
-    float acc = 0.f;
-    const int k1 = A.inv_start[g + 1];
-    for (int k = A.inv_start[g]; k < k1; ++k)
-      acc = acc + A.r[(size_t(k) * NC + c) * S + s];
-    const float a = __fmul_rn(acc, A.minv[gc]);
-    float vv = newmark_correct(A.v[i], a, A.dt2);
-    float uu = A.u[i];
-    if (A.predict) newmark_predict(uu, vv, a, A.dt, A.dt2, A.dtsq2);
-    A.u[i] = uu;
-    A.v[i] = vv;
-    if (A.a_store) A.a_store[i] = a;
-    bad |= !isfinite(uu);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const int g = i / SV, s = (i - g * SV) * V;
+    const size_t o = size_t(g) * NC * S + s;
+    const int k0 = A.inv_start[g], k1 = A.inv_start[g + 1];
+    ShotVec<V> u[NC], v[NC], acc[NC];
+    float mi[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      u[c] = ld_shots<V>(A.u + o + size_t(c) * S);
+      v[c] = ld_shots<V>(A.v + o + size_t(c) * S);
+      mi[c] = A.minv[size_t(g) * NC + c];
+#pragma unroll
+      for (int w = 0; w < V; ++w) acc[c].x[w] = 0.f;
+    }
+    for (int k = k0; k < k1; ++k) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const ShotVec<V> t = ld_shots<V>(A.r + (size_t(k) * NC + c) * S + s);
+#pragma unroll
+        for (int w = 0; w < V; ++w) acc[c].x[w] = acc[c].x[w] + t.x[w];
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      ShotVec<V> a;
+#pragma unroll
+      for (int w = 0; w < V; ++w) {
+        a.x[w] = __fmul_rn(acc[c].x[w], mi[c]);
+        v[c].x[w] = newmark_correct(v[c].x[w], a.x[w], A.dt2);
+        if (A.predict) newmark_predict(u[c].x[w], v[c].x[w], a.x[w], A.dt, A.dt2, A.dtsq2);
+        bad |= !isfinite(u[c].x[w]);
+      }
+      if (A.predict) st_shots<V>(A.u + o + size_t(c) * S, u[c]);
+      st_shots<V>(A.v + o + size_t(c) * S, v[c]);
+      if (A.a_store) st_shots<V>(A.a_store + o + size_t(c) * S, a);
+    }
   }
   if (bad) *A.flag = 1;
   if (A.advance && blockIdx.x == 0 && threadIdx.x == 0) *A.step += 1;
@@ -336,194 +385,187 @@ __global__ void __launch_bounds__(NP * 8) k_stiffness_batched4(BatchArgs A, int 
   }
 }
 
-// Row form of k_stiffness_batched4 (owner-computes): one thread per element
-// row (five points, iz fixed) and quad of shots; EB elements x 5 rows x T
-// quads per block.  The xi-direction contractions of the gradient and of the
-// divergence run on the row held in registers (warp-uniform coefficients);
-// the gamma-direction ones read columns of the element's displacement and F1
-// in shared memory.  Per shot the operations and their order are those of
-// k_stiffness_batched4 (same bits).  Dynamic shared memory: EB x NC x 2 x 25
-// x T float4.
-template <int NC, int EB>
-__global__ void __launch_bounds__(EB * NG * 8, EB <= 4 ? 3 : 2) k_stiffness_batched4r(BatchArgs A, int T) {
-  extern __shared__ __align__(16) float4 dynb[];
-  // the block's Jacobian and material words [EB][7][25], loaded once by all threads
-  __shared__ float sgeo[EB * 7 * NP];
-  const int rowq = threadIdx.x / T, j = threadIdx.x - rowq * T;
-  const int le = rowq / NG, iz = rowq - le * NG;
-  const int shot0 = (blockIdx.y * T + j) * 4;
-  const int e = blockIdx.x * EB + le;
-  const bool act = shot0 < A.S && e < A.nspec_b;
-  float4 *su = dynb + size_t(le) * NC * 2 * NP * T;   // [c][25][T]
-  float4 *sF1 = su + NC * NP * T;                     // [c][25][T]
-  for (int i = threadIdx.x; i < EB * NP; i += blockDim.x) {
-    const int ee = i / NP, q = i - ee * NP;
-    const int eg = blockIdx.x * EB + ee;
-    const size_t pg = size_t(eg < A.nspec_b ? eg : 0) * NP + q;
-    float *d = sgeo + ee * 7 * NP + q;
-    d[0] = __ldg(A.xix + pg); d[NP] = __ldg(A.xiz + pg); d[2 * NP] = __ldg(A.gax + pg);
-    d[3 * NP] = __ldg(A.gaz + pg); d[4 * NP] = __ldg(A.jac + pg);
-    d[5 * NP] = __ldg(A.prop0 + pg); d[6 * NP] = __ldg(A.prop1 + pg);
+// Thread form of the owner-computes batched element kernel: one thread per
+// element and shot, the element's 25 points in registers.  The lanes of a
+// warp are the shots of one element (of 32 / G elements when the shots fill
+// only G < 32 lanes), so every field access is coalesced over shots and the
+// contractions need neither shared memory nor barriers: the xi derivatives
+// replace the displacement row by row, the gamma derivatives are formed
+// column by column, F0 and F1 replace them, and the divergence contracts F0
+// rows and F1 columns in place (two components paired in FFMA2, which rounds
+// each lane as fmaf).  The block's index, slot, geometry and material words
+// are staged once in shared memory and read as broadcasts.  GEO 1, MAT 1: as
+// in the row kernel, words that are one value an element come from its record.
+// The row form read every gamma column from shared memory once a row (63% of
+// the L1's wavefronts, 122 instructions a point of 32 shots); this form
+// executes about half.  Per shot the operations and their order are those of
+// k_stiffness_batched (same bits).
+template <int GEO, int MAT>
+constexpr int bt_words() { return 2 + (GEO ? 0 : 5) + (MAT ? 0 : 2); }   // staged words a point
+
+// One component pair (P-SV) or one component (SH) of a thread's shot.
+template <int NC> struct BtV;
+template <> struct BtV<2> { float2 v; };
+template <> struct BtV<1> { float v; };
+__device__ __forceinline__ void bt_fma(BtV<2> &a, float h, const BtV<2> &x) { a.v = fma2(f2(h), x.v, a.v); }
+__device__ __forceinline__ void bt_fma(BtV<1> &a, float h, const BtV<1> &x) { a.v = fmaf(h, x.v, a.v); }
+__device__ __forceinline__ void bt_zero(BtV<2> &a) { a.v = make_float2(0.f, 0.f); }
+__device__ __forceinline__ void bt_zero(BtV<1> &a) { a.v = 0.f; }
+template <int NC>
+__device__ __forceinline__ float bt_get(const BtV<NC> &a, int c);
+template <>
+__device__ __forceinline__ float bt_get<2>(const BtV<2> &a, int c) { return c ? a.v.y : a.v.x; }
+template <>
+__device__ __forceinline__ float bt_get<1>(const BtV<1> &a, int) { return a.v; }
+
+// out_i = sum_l coef(i, l) x_l over the five values of a line, in place; DIV:
+// the divergence's weighted derivatives hpw[l*5+i], else hp[i*5+l].
+template <int NC, bool DIV>
+__device__ __forceinline__ void bt_line(BtV<NC> &x0, BtV<NC> &x1, BtV<NC> &x2, BtV<NC> &x3, BtV<NC> &x4) {
+  const BtV<NC> x[NG] = {x0, x1, x2, x3, x4};
+  BtV<NC> o[NG];
+#pragma unroll
+  for (int i = 0; i < NG; ++i) {
+    bt_zero(o[i]);
+#pragma unroll
+    for (int l = 0; l < NG; ++l) bt_fma(o[i], DIV ? c_hpw[l * NG + i] : c_hp[i * NG + l], x[l]);
   }
-  const size_t pe = size_t(act ? e : 0) * NP + iz * NG;
-  int g[NG];
-  float4 ur[NC][NG];
-#pragma unroll
-  for (int ix = 0; ix < NG; ++ix) g[ix] = act ? __ldg(A.ibool + pe + ix) : 0;
-#pragma unroll
-  for (int ix = 0; ix < NG; ++ix)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      ur[c][ix] = act ? *reinterpret_cast<const float4 *>(A.u + (size_t(g[ix]) * NC + c) * A.S + shot0)
-                      : make_float4(0.f, 0.f, 0.f, 0.f);
-      su[(c * NP + iz * NG + ix) * T + j] = ur[c][ix];
-    }
-  float hz[NG];
-#pragma unroll
-  for (int l = 0; l < NG; ++l) hz[l] = c_hp[iz * NG + l];
-  __syncthreads();
-  // xi-direction derivatives of the row's five points, in place of the row
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    float4 dx[NG];
-#pragma unroll
-    for (int ix = 0; ix < NG; ++ix) {
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        float d = 0.f;
-#pragma unroll
-        for (int l = 0; l < NG; ++l) d = fmaf(c_hp[ix * NG + l], (&ur[c][l].x)[w], d);
-        (&dx[ix].x)[w] = d;
+  x0 = o[0]; x1 = o[1]; x2 = o[2]; x3 = o[3]; x4 = o[4];
+}
+
+constexpr int BT_THREADS = 128;
+
+// G lanes per element (a power of two, at least the shots of the tile or 32).
+template <int NC, int GEO, int MAT>
+__global__ void __launch_bounds__(BT_THREADS, 4) k_stiffness_batched_t(BatchArgs A, int G) {
+  extern __shared__ __align__(16) float btsm[];
+  const int NE = BT_THREADS / G;                  // elements of the block
+  const int NPB = NE * NP;
+  const int e0 = blockIdx.x * NE;
+  {
+    const size_t p0 = size_t(e0) * NP;
+    const int n = min(NE, A.nspec_b - e0) * NP;
+    int *si = reinterpret_cast<int *>(btsm);
+    for (int i = threadIdx.x; i < n; i += BT_THREADS) {
+      si[i] = __ldg(A.ibool + p0 + i);
+      si[NPB + i] = __ldg(A.slot + p0 + i);
+      int w = 2;
+      if (GEO == 0) {
+        btsm[w++ * NPB + i] = __ldg(A.xix + p0 + i);
+        btsm[w++ * NPB + i] = __ldg(A.xiz + p0 + i);
+        btsm[w++ * NPB + i] = __ldg(A.gax + p0 + i);
+        btsm[w++ * NPB + i] = __ldg(A.gaz + p0 + i);
+        btsm[w++ * NPB + i] = __ldg(A.jac + p0 + i);
       }
-    }
-#pragma unroll
-    for (int ix = 0; ix < NG; ++ix) ur[c][ix] = dx[ix];
-  }
-  // per point: gamma-direction derivatives from the columns, stress, F; F0
-  // replaces the xi derivatives in registers, F1 goes to shared memory
-#pragma unroll
-  for (int ix = 0; ix < NG; ++ix) {
-    const float *gw = sgeo + le * 7 * NP + iz * NG + ix;
-    const float xix = gw[0], xiz = gw[NP], gax = gw[2 * NP], gaz = gw[3 * NP], jac = gw[4 * NP];
-    const float c0 = gw[5 * NP], mu = gw[6 * NP];
-    float4 dg[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        float d = 0.f;
-#pragma unroll
-        for (int l = 0; l < NG; ++l) d = fmaf(hz[l], (&su[(c * NP + l * NG + ix) * T + j].x)[w], d);
-        (&dg[c].x)[w] = d;
+      if (MAT == 0) {
+        btsm[w++ * NPB + i] = __ldg(A.prop0 + p0 + i);
+        btsm[w++ * NPB + i] = __ldg(A.prop1 + p0 + i);
       }
-    }
-    float4 f0[NC], f1[NC];
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      float dxi[NC], dga[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        dxi[c] = (&ur[c][ix].x)[w];
-        dga[c] = (&dg[c].x)[w];
-      }
-      float Sx[NC], Sz[NC];
-      if (NC == 2) {
-        const float du00 = xix * dxi[0] + gax * dga[0], du01 = xiz * dxi[0] + gaz * dga[0];
-        const float du10 = xix * dxi[NC - 1] + gax * dga[NC - 1];
-        const float du11 = xiz * dxi[NC - 1] + gaz * dga[NC - 1];
-        const float lam = c0 - 2.f * mu;
-        const float sxx = c0 * du00 + lam * du11;
-        const float szz = c0 * du11 + lam * du00;
-        const float sxz = mu * (du01 + du10);
-        Sx[0] = sxx; Sz[0] = sxz; Sx[NC - 1] = sxz; Sz[NC - 1] = szz;
-      } else {
-        Sx[0] = mu * (xix * dxi[0] + gax * dga[0]);
-        Sz[0] = mu * (xiz * dxi[0] + gaz * dga[0]);
-      }
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        (&f0[c].x)[w] = jac * (Sx[c] * xix + Sz[c] * xiz);
-        (&f1[c].x)[w] = jac * (Sx[c] * gax + Sz[c] * gaz);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      ur[c][ix] = f0[c];
-      sF1[(c * NP + iz * NG + ix) * T + j] = f1[c];
     }
   }
-  const int bs = act ? __ldg(A.bc_slot + e) : -1;
-  const int src = act ? __ldg(A.src_head + e) : -1;
-  float wz[NG];
-#pragma unroll
-  for (int l = 0; l < NG; ++l) wz[l] = c_hpw[l * NG + iz];
-  const float wiz = c_w[iz];
+  const int le = threadIdx.x / G, shot = blockIdx.y * 32 + (threadIdx.x - le * G);
+  const int e = e0 + le;
+  const bool act = e < A.nspec_b && shot < A.S;
+  float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 m2 = make_float2(0.f, 0.f);
+  if (GEO == 1 && act) g4 = __ldg(reinterpret_cast<const float4 *>(A.erec + size_t(e) * 8));
+  if (MAT == 1 && act) m2 = __ldg(reinterpret_cast<const float2 *>(A.erec + size_t(e) * 8 + 4));
   __syncthreads();
   if (!act) return;
+  const int *sg = reinterpret_cast<const int *>(btsm) + le * NP, *ss = sg + NPB;
+  const float *sw = btsm + 2 * NPB + le * NP;
+  BtV<NC> U[NP], D[NP];
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    const float *u = A.u + size_t(sg[q]) * NC * A.S + shot;
+    if constexpr (NC == 2) U[q].v = make_float2(u[0], u[A.S]);
+    else U[q].v = u[0];
+  }
 #pragma unroll
   for (int ix = 0; ix < NG; ++ix) {
-    const int q = iz * NG + ix;
-    float a[NC][4];
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
+    for (int iz = 0; iz < NG; ++iz) D[iz * NG + ix] = U[iz * NG + ix];
+    bt_line<NC, false>(D[ix], D[5 + ix], D[10 + ix], D[15 + ix], D[20 + ix]);
+  }
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        float t1 = 0.f, t2 = 0.f;
+  for (int iz = 0; iz < NG; ++iz) bt_line<NC, false>(U[5 * iz], U[5 * iz + 1], U[5 * iz + 2], U[5 * iz + 3], U[5 * iz + 4]);
 #pragma unroll
-        for (int l = 0; l < NG; ++l) {
-          t1 = fmaf((&ur[c][l].x)[w], c_hpw[l * NG + ix], t1);
-          t2 = fmaf((&sF1[(c * NP + l * NG + ix) * T + j].x)[w], wz[l], t2);
-        }
-        a[c][w] = -(wiz * t1 + c_w[ix] * t2);
-      }
+  for (int q = 0; q < NP; ++q) {
+    float xix, xiz = 0.f, gax = 0.f, gaz, jac;
+    if (GEO == 1) { xix = g4.x; gaz = g4.y; jac = g4.z; }
+    else { xix = sw[q]; xiz = sw[NPB + q]; gax = sw[2 * NPB + q]; gaz = sw[3 * NPB + q]; jac = sw[4 * NPB + q]; }
+    float c0, mu;
+    if (MAT == 1) { c0 = m2.x; mu = m2.y; }
+    else { c0 = sw[(GEO ? 0 : 5) * NPB + q]; mu = sw[(GEO ? 1 : 6) * NPB + q]; }
+    // x + 0 and x * 0 of the rectangle's zero words change no bit
+    auto ddx = [&](float dxi, float dga) { return GEO ? xix * dxi : xix * dxi + gax * dga; };
+    auto ddz = [&](float dxi, float dga) { return GEO ? gaz * dga : xiz * dxi + gaz * dga; };
+    auto f0 = [&](float sx, float sz) { return GEO ? jac * (sx * xix) : jac * (sx * xix + sz * xiz); };
+    auto f1 = [&](float sx, float sz) { return GEO ? jac * (sz * gaz) : jac * (sx * gax + sz * gaz); };
+    if constexpr (NC == 2) {
+      const float2 dx = U[q].v, dg = D[q].v;
+      const float du00 = ddx(dx.x, dg.x), du01 = ddz(dx.x, dg.x), du10 = ddx(dx.y, dg.y), du11 = ddz(dx.y, dg.y);
+      const float lam = c0 - 2.f * mu;
+      const float sxx = c0 * du00 + lam * du11;
+      const float szz = c0 * du11 + lam * du00;
+      const float sxz = mu * (du01 + du10);
+      U[q].v = make_float2(f0(sxx, sxz), f0(sxz, szz));
+      D[q].v = make_float2(f1(sxx, sxz), f1(sxz, szz));
+    } else {
+      const float sx = mu * ddx(U[q].v, D[q].v), sz = mu * ddz(U[q].v, D[q].v);
+      U[q].v = f0(sx, sz);
+      D[q].v = f1(sx, sz);
     }
+  }
+#pragma unroll
+  for (int iz = 0; iz < NG; ++iz) bt_line<NC, true>(U[5 * iz], U[5 * iz + 1], U[5 * iz + 2], U[5 * iz + 3], U[5 * iz + 4]);
+#pragma unroll
+  for (int ix = 0; ix < NG; ++ix) bt_line<NC, true>(D[ix], D[5 + ix], D[10 + ix], D[15 + ix], D[20 + ix]);
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    const int iz = q / NG, ix = q - iz * NG;
+    float *r = A.r + size_t(ss[q]) * NC * A.S + shot;
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+      r[size_t(c) * A.S] = -(c_w[iz] * bt_get<NC>(U[q], c) + c_w[ix] * bt_get<NC>(D[q], c));
+  }
+  const int bs = __ldg(A.bc_slot + e), src = __ldg(A.src_head + e);
+  if (bs < 0 && src < 0) return;
+  // boundary and source elements: the Stacey traction, then the sources, onto
+  // the thread's own results
+  const int step = *A.step;
+  for (int q = 0; q < NP; ++q) {
+    float *r = A.r + size_t(ss[q]) * NC * A.S + shot;
+    const size_t g = size_t(sg[q]) * NC;
+    float a[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) a[c] = r[size_t(c) * A.S];
     if (bs >= 0) {
       const size_t k = size_t(bs) * NP + q;
       const float wq = A.bc_w[k];
       if (wq != 0.f) {
         const float nx = A.bc_nx[k], nz = A.bc_nz[k], j1 = A.bc_j1[k];
         if (NC == 2) {
-          const float4 vx4 = *reinterpret_cast<const float4 *>(A.v + (size_t(g[ix]) * NC) * A.S + shot0);
-          const float4 vz4 = *reinterpret_cast<const float4 *>(A.v + (size_t(g[ix]) * NC + NC - 1) * A.S + shot0);
+          const float vx = A.v[g * A.S + shot], vz = A.v[(g + NC - 1) * A.S + shot];
           const float rvp = A.bc_imp0[k], rvs = A.bc_imp1[k];
-#pragma unroll
-          for (int w = 0; w < 4; ++w) {
-            const float vx = (&vx4.x)[w], vz = (&vz4.x)[w];
-            const float vn = vx * nx + vz * nz;
-            const float fx = ((vn * nx / (j1 * j1)) * (rvp - rvs)) + vx * rvs;
-            const float fz = ((vn * nz / (j1 * j1)) * (rvp - rvs)) + vz * rvs;
-            a[0][w] += -1.f * fx * j1 * wq;
-            a[NC - 1][w] += -1.f * fz * j1 * wq;
-          }
+          const float vn = vx * nx + vz * nz;
+          const float fx = ((vn * nx / (j1 * j1)) * (rvp - rvs)) + vx * rvs;
+          const float fz = ((vn * nz / (j1 * j1)) * (rvp - rvs)) + vz * rvs;
+          a[0] += -1.f * fx * j1 * wq;
+          a[NC - 1] += -1.f * fz * j1 * wq;
         } else {
-          const float4 v4 = *reinterpret_cast<const float4 *>(A.v + size_t(g[ix]) * A.S + shot0);
-#pragma unroll
-          for (int w = 0; w < 4; ++w) a[0][w] += -1.f * (wq * j1) * A.bc_imp1[k] * (&v4.x)[w];
+          a[0] += -1.f * (wq * j1) * A.bc_imp1[k] * A.v[g * A.S + shot];
         }
       }
     }
-    if (src >= 0) {
-      const int step = *A.step;
-      for (int s = src; s >= 0; s = A.src_next[s]) {
-        const int ws = A.src_shot[s] - shot0;
-        if (ws < 0 || ws > 3) continue;
-        const float f = step < A.nstep ? A.stf[size_t(step) * A.nsrc + s] : 0.f;
+    for (int s = src; s >= 0; s = A.src_next[s]) {
+      if (A.src_shot[s] != shot) continue;
+      const float f = step < A.nstep ? A.stf[size_t(step) * A.nsrc + s] : 0.f;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const float add = f * A.src_arr[(size_t(s) * 2 + c) * NP + q];
-          // sources in chain order, as the one-shot kernel adds them
-          if (ws == 0) a[c][0] += add;
-          else if (ws == 1) a[c][1] += add;
-          else if (ws == 2) a[c][2] += add;
-          else a[c][3] += add;
-        }
-      }
+      for (int c = 0; c < NC; ++c) a[c] += f * A.src_arr[(size_t(s) * 2 + c) * NP + q];
     }
-    const int sl = __ldg(A.slot + pe + ix);
 #pragma unroll
-    for (int c = 0; c < NC; ++c)
-      *reinterpret_cast<float4 *>(A.r + (size_t(sl) * NC + c) * A.S + shot0) =
-          make_float4(a[c][0], a[c][1], a[c][2], a[c][3]);
+    for (int c = 0; c < NC; ++c) r[size_t(c) * A.S] = a[c];
   }
 }
 
@@ -549,40 +591,6 @@ __global__ void __launch_bounds__(256) k_update_batched4(UpdateArgs A, int S) {
     if (A.predict) reinterpret_cast<float4 *>(A.u)[i] = uu;
     reinterpret_cast<float4 *>(A.v)[i] = vv;
     reinterpret_cast<float4 *>(A.accum)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (A.a_store) reinterpret_cast<float4 *>(A.a_store)[i] = make_float4(a[0], a[1], a[2], a[3]);
-  }
-  if (bad) *A.flag = 1;
-  if (A.advance && blockIdx.x == 0 && threadIdx.x == 0) *A.step += 1;
-}
-
-__global__ void __launch_bounds__(256) k_update_batched4_gather(UpdateArgs A, int S, int NC) {
-  const int n4 = A.n >> 2;
-  const int stride = gridDim.x * blockDim.x;
-  bool bad = false;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
-    const int s = (4 * i) % S;
-    const int gc = (4 * i) / S;
-    const int g = gc / NC, c = gc - g * NC;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int k1 = A.inv_start[g + 1];
-    for (int k = A.inv_start[g]; k < k1; ++k) {
-      const float4 t = *reinterpret_cast<const float4 *>(A.r + (size_t(k) * NC + c) * S + s);
-      acc.x = acc.x + t.x; acc.y = acc.y + t.y; acc.z = acc.z + t.z; acc.w = acc.w + t.w;
-    }
-    const float mi = A.minv[gc];
-    float4 uu = reinterpret_cast<float4 *>(A.u)[i];
-    float4 vv = reinterpret_cast<float4 *>(A.v)[i];
-    float *pc = &acc.x, *pu = &uu.x, *pv = &vv.x;
-    float a[4];
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      a[w] = __fmul_rn(pc[w], mi);
-      pv[w] = newmark_correct(pv[w], a[w], A.dt2);
-      if (A.predict) newmark_predict(pu[w], pv[w], a[w], A.dt, A.dt2, A.dtsq2);
-      bad |= !isfinite(pu[w]);
-    }
-    if (A.predict) reinterpret_cast<float4 *>(A.u)[i] = uu;
-    reinterpret_cast<float4 *>(A.v)[i] = vv;
     if (A.a_store) reinterpret_cast<float4 *>(A.a_store)[i] = make_float4(a[0], a[1], a[2], a[3]);
   }
   if (bad) *A.flag = 1;
@@ -631,11 +639,13 @@ __global__ void __launch_bounds__(32) k_receivers_batched(RecArgs A, int S) {
         float x[32];
 #pragma unroll
         for (int q = 0; q < 32; ++q) x[q] = 0.f;
+#pragma unroll
         for (int q = 0; q < NP; ++q) {
           const int g = A.ibool[size_t(ce) * NP + q];
           const size_t k = (size_t(g) * NC + c) * S + shot;
           float sum = 0.f;
-          if (A.cpl.inv_start) {
+          if (A.types[t] == 0) {                 // displacement: no sum
+          } else if (A.cpl.inv_start) {
             for (int j = A.cpl.inv_start[g]; j < A.cpl.inv_start[g + 1]; ++j)
               sum = sum + A.cpl.r[(size_t(j) * NC + c) * S + shot];
           } else {

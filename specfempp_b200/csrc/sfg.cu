@@ -240,7 +240,6 @@ struct sfg_handle {
   sfg::dev::TileArgs tile_layout{};
   sfg::dev::TileBArgs tileb_layout{};   // batched shots
   int tile_smem = 0, tile_blocks_per_sm = 0;
-  bool b4r_attr = false;                 // shared-memory attribute of the row-form batched kernel set
   bool btile_ok = false;                 // batched tiles of four elements (variant 7) built
   void *flush_buf = nullptr;
   size_t flush_bytes = 0;
@@ -558,6 +557,7 @@ void launch_stiffness_batched(sfg_handle *h, const DevMedium &el, const int *ste
   B.nsrc = h->asmb.nsrc; B.nstep = h->asmb.nstep;
   B.step = step;
   B.u = el.u; B.v = el.v; B.accum = el.accum; B.r = el.r; B.slot = el.slot;
+  B.erec = el.erec;
   B.S = el.S;
   // quad-shot kernels when the shots come in fours
   const bool quad = el.S % 4 == 0;
@@ -583,21 +583,28 @@ void launch_stiffness_batched(sfg_handle *h, const DevMedium &el, const int *ste
       else sfg::dev::k_stiffness_batched<1, false><<<grid, threads, 0, s>>>(B);
     }
   };
-  if (variant == 4 && quad) {
-    // owner-computes with the row-form element kernel (4 elements per block)
-    constexpr int EB = 4;
+  if (variant == 4) {
+    // owner-computes with one thread per element and shot: G lanes an element
     B.nspec_b = el.nspec;
-    const int smem = EB * el.ncomp * 2 * sfg::dev::NP * T * int(sizeof(float4));
-    if (!h->b4r_attr) {
-      SFG_CUDA(cudaFuncSetAttribute(sfg::dev::k_stiffness_batched4r<2, EB>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, EB * 2 * 2 * 25 * 8 * 16));
-      SFG_CUDA(cudaFuncSetAttribute(sfg::dev::k_stiffness_batched4r<1, EB>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, EB * 1 * 2 * 25 * 8 * 16));
-      h->b4r_attr = true;
-    }
-    const dim3 grid((el.nspec + EB - 1) / EB, tiles);
-    if (el.ncomp == 2) sfg::dev::k_stiffness_batched4r<2, EB><<<grid, EB * sfg::dev::NG * T, smem, s>>>(B, T);
-    else sfg::dev::k_stiffness_batched4r<1, EB><<<grid, EB * sfg::dev::NG * T, smem, s>>>(B, T);
+    int G = 2;
+    while (G < 32 && G < el.S) G *= 2;
+    const int ne = sfg::dev::BT_THREADS / G;
+    const dim3 grid((el.nspec + ne - 1) / ne, (el.S + 31) / 32);
+    auto go = [&](auto kern, int words) {
+      const int smem = words * ne * sfg::dev::NP * int(sizeof(float));
+      SFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      kern<<<grid, sfg::dev::BT_THREADS, smem, s>>>(B, G);
+    };
+    const bool geo = h->asmb.el.row.straight, mat = h->asmb.el.row.matconst;
+    auto pick = [&](auto nc) {
+      constexpr int NC = decltype(nc)::value;
+      if (geo && mat) go(sfg::dev::k_stiffness_batched_t<NC, 1, 1>, sfg::dev::bt_words<1, 1>());
+      else if (geo) go(sfg::dev::k_stiffness_batched_t<NC, 1, 0>, sfg::dev::bt_words<1, 0>());
+      else if (mat) go(sfg::dev::k_stiffness_batched_t<NC, 0, 1>, sfg::dev::bt_words<0, 1>());
+      else go(sfg::dev::k_stiffness_batched_t<NC, 0, 0>, sfg::dev::bt_words<0, 0>());
+    };
+    if (el.ncomp == 2) pick(std::integral_constant<int, 2>{});
+    else pick(std::integral_constant<int, 1>{});
     return;
   }
   if (variant >= 3) {
@@ -828,10 +835,20 @@ void launch_update(sfg_handle *h, int medium, bool predict, bool advance, cudaSt
     return;
   }
   if (h->variant >= 3) {
-    if (D.S > 1 && D.S % 4 == 0)
-      sfg::dev::k_update_batched4_gather<<<grid_for(U.n / 4), 256, 0, s>>>(U, D.S, D.ncomp);
-    else if (D.S > 1) sfg::dev::k_update_batched_gather<<<grid_for(U.n), 256, 0, s>>>(U, D.S, D.ncomp);
-    else if (D.ncomp == 2) sfg::dev::k_update_gather<2><<<grid_for(U.n / 2), 256, 0, s>>>(U);
+    if (D.S > 1) {
+      const int V = D.S % 4 == 0 ? 4 : (D.S % 2 == 0 ? 2 : 1);
+      const int grid = grid_for(U.n / (V * D.ncomp));
+      auto go = [&](auto kern) { kern<<<grid, 256, 0, s>>>(U, D.S); };
+      if (D.ncomp == 2) {
+        if (V == 4) go(sfg::dev::k_update_batched_gather<2, 4>);
+        else if (V == 2) go(sfg::dev::k_update_batched_gather<2, 2>);
+        else go(sfg::dev::k_update_batched_gather<2, 1>);
+      } else {
+        if (V == 4) go(sfg::dev::k_update_batched_gather<1, 4>);
+        else if (V == 2) go(sfg::dev::k_update_batched_gather<1, 2>);
+        else go(sfg::dev::k_update_batched_gather<1, 1>);
+      }
+    } else if (D.ncomp == 2) sfg::dev::k_update_gather<2><<<grid_for(U.n / 2), 256, 0, s>>>(U);
     else sfg::dev::k_update_gather<1><<<grid_for(U.n), 256, 0, s>>>(U);
     return;
   }
@@ -1505,15 +1522,13 @@ void autotune(sfg_handle *h) {
   if (h->variant == 6 && h->epb != 16) h->epb = 32;
   if (h->variant == 7 && !h->btile_ok) h->variant = 3;   // batched tiles of four elements
   if (h->asmb.nshots > 1 && h->variant == 2) h->variant = 1;  // no persistent batched kernel
-  // batched: variant 4 is owner-computes with the row-form element kernel (shots in fours)
-  if (h->asmb.nshots > 1 && h->variant == 4 && h->asmb.nshots % 4 != 0) h->variant = 3;
   const bool special = h->el.aniso || h->el.ncomp >= 3;   // anisotropic, Cosserat or poroelastic
   if (special && h->variant == 2) h->variant = 1;
   if (special && h->variant == 4) h->variant = 3;
   std::vector<std::pair<int, int>> cand;
   if (h->asmb.nshots > 1) {
     for (int v : {1, 3, 4})
-      if ((!fix_v || v == h->variant) && (v != 4 || h->asmb.nshots % 4 == 0)) cand.push_back({v, 16});
+      if (!fix_v || v == h->variant) cand.push_back({v, 16});
     if (h->tile_ok && (!fix_v || h->variant == 5)) cand.push_back({5, 16});
     if (h->btile_ok && (!fix_v || h->variant == 7)) cand.push_back({7, 16});
   } else {
@@ -2394,7 +2409,7 @@ int sfg_set_model2d(sfg_handle *h, const float *rho, const float *kappa, const f
         put(D.erec, M.row.erec);
       }
       // the step graphs hold the element kernel of the old model's class
-      if (row_matconst(h) != mat0 && h->variant == 6) recapture(h);
+      if (row_matconst(h) != mat0 && (h->variant == 6 || (h->asmb.nshots > 1 && h->variant == 4))) recapture(h);
       refresh_tile_records(h);
       if (h->adj.st_c && !h->asmb.el.stacey_c.empty())
         SFG_CUDA(cudaMemcpy(h->adj.st_c, h->asmb.el.stacey_c.data(), h->asmb.el.stacey_c.size() * sizeof(float),
