@@ -76,6 +76,18 @@ __device__ __forceinline__ int ld_dep(const int *p) {
   asm volatile("ld.global.s32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
   return x;
 }
+// the same past the L1 (for loads before the wait, of data that is complete
+// but that another SM wrote)
+__device__ __forceinline__ float ld_l2(const float *p) {
+  float x;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(x) : "l"(p) : "memory");
+  return x;
+}
+__device__ __forceinline__ float2 ld_l22(const float *p) {
+  float2 x;
+  asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "l"(p) : "memory");
+  return x;
+}
 __device__ __forceinline__ float2 ld_dep2(const float *p) {
   float2 x;
   asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "l"(p) : "memory");
@@ -118,6 +130,7 @@ struct MedArgs {
 };
 
 struct RecArgs;
+struct SegRecord;
 
 struct StiffArgs {
   MedArgs el, ac;
@@ -125,6 +138,10 @@ struct StiffArgs {
   // first rec_blocks blocks, one warp each: acoustic ones first
   const RecArgs *rec_ac, *rec_el;
   int nrec_ac, nrec_el, rec_blocks;
+  // recording step (adjoint): the save_blocks blocks after those store the
+  // predicted velocity at the Stacey points and the step's segment slot
+  SegRecord *save_el, *save_ac;
+  int save_blocks;
   const int *__restrict__ src_next;
   const float *__restrict__ src_arr;   // [nsrc][2][25]
   const float *__restrict__ src_arr2;  // poroelastic fluid rows [nsrc][2][25] (else null)
@@ -491,13 +508,21 @@ __device__ __noinline__ void receiver_blocks(const RecArgs *ac, const RecArgs *e
   else receiver_warp<true>(*el, i - nac, lane, smem + w * 3 * NP);
 }
 
+__device__ void save_stacey_velocity(const StiffArgs &S);
+
+// The blocks of a launch before its element blocks.
+__device__ __forceinline__ void leading_block(const StiffArgs &S, float *smem) {
+  if (int(blockIdx.x) < S.rec_blocks) receiver_blocks(S.rec_ac, S.rec_el, S.nrec_ac, S.nrec_el, smem);
+  else save_stacey_velocity(S);
+}
+
 template <int E, int EK, bool LOCAL>
 __global__ void __launch_bounds__(NP * E, 64 / ((NP * E + 31) / 32)) k_stiffness(StiffArgs S) {
   __shared__ __align__(16) unsigned char smem[sizeof(float) * NP * E * (EK == 4 ? 12 : EK == 3 ? 9 : 6)];
   __shared__ float shp[NP], shpw[NP], sw[NG];
-  const int b = int(blockIdx.x) - S.rec_blocks;
+  const int b = int(blockIdx.x) - S.rec_blocks - S.save_blocks;
   if (LOCAL && b < 0) {
-    receiver_blocks(S.rec_ac, S.rec_el, S.nrec_ac, S.nrec_el, reinterpret_cast<float *>(smem));
+    leading_block(S, reinterpret_cast<float *>(smem));
     return;
   }
   load_quad(S.quad, shp, shpw, sw, threadIdx.x);
@@ -709,9 +734,30 @@ struct SegRecord {
   float *vst;
   size_t vstride;
   const int *st_pt;
-  int nst;
-  int i;          // next step of the segment (k0 + i)
+  int nst, nc;    // Stacey points, components of the medium
+  const float *v; // the medium's velocity
+  // chained steps: the slot of the step being taken, written by its element
+  // launch; else the next step of the segment (k0 + i)
+  int i;
 };
+
+__device__ __noinline__ void save_stacey(SegRecord *rec, int step, int b, int nb) {
+  const int i = step - rec->k0, n = rec->nst * rec->nc, nc = rec->nc;
+  float *dst = rec->vst + size_t(i) * rec->vstride;
+  for (int t = b * blockDim.x + threadIdx.x; t < n; t += nb * blockDim.x) {
+    const int j = t / nc, c = t - j * nc;
+    dst[t] = ld_dep(rec->v + size_t(rec->st_pt[j]) * nc + c);
+  }
+  if (b == 0 && threadIdx.x == 0) rec->i = i;
+}
+
+__device__ __forceinline__ void save_stacey_velocity(const StiffArgs &S) {
+  pdl_wait();
+  pdl_release();
+  const int step = ld_dep(S.step), b = int(blockIdx.x) - S.rec_blocks;
+  if (S.save_el) save_stacey(S.save_el, step, b, S.save_blocks);
+  if (S.save_ac) save_stacey(S.save_ac, step, b, S.save_blocks);
+}
 
 struct UpdateArgs {
   float *__restrict__ u, *__restrict__ v, *__restrict__ accum;
@@ -737,7 +783,8 @@ struct UpdateArgs {
   int *flag;                     // set to 1 on a non-finite displacement
   int *step;
   int advance;                   // increment the step counter (last update of a step)
-  const SegRecord *rec;          // optional segment recording (then advance = 0)
+  const SegRecord *rec;          // optional segment recording
+  int rec_chain;                 // its slot is rec->i (chained steps), else the step's (then advance = 0)
 };
 
 __device__ __forceinline__ float coupling_entry(const UpdateArgs &A, int k, int comp) {
@@ -798,7 +845,7 @@ __global__ void __launch_bounds__(256) k_update(UpdateArgs A) {
 #pragma unroll
     for (int c = 0; c < 4; ++c) a[c] = __fmul_rn(pa[c], pm[c]);
     if (A.rec) {
-      const size_t off = size_t(*A.step - A.rec->k0) * A.rec->stride;
+      const size_t off = size_t(*A.step - A.rec->k0) * A.rec->stride;   // never chained
       reinterpret_cast<float4 *>(A.rec->u + off)[i] = uu;
       reinterpret_cast<float4 *>(A.rec->a + off)[i] = make_float4(a[0], a[1], a[2], a[3]);
     }
@@ -820,7 +867,7 @@ __global__ void __launch_bounds__(256) k_update(UpdateArgs A) {
     float vv = newmark_correct(A.v[i], a, A.dt2);
     float uu = A.u[i];
     if (A.rec) {
-      const size_t off = size_t(*A.step - A.rec->k0) * A.rec->stride;
+      const size_t off = size_t(*A.step - A.rec->k0) * A.rec->stride;   // never chained
       A.rec->u[off + i] = uu;
       A.rec->a[off + i] = a;
     }
@@ -856,14 +903,14 @@ __device__ __forceinline__ PointPre<NC> update_point_pre(const UpdateArgs &A, in
   P.k1 = A.inv_start[g + 1];
   if (NC > 2) return P;      // u, v and M^-1 after the sum: fewer registers, more warps
   if (NC == 2) {
-    const float2 u2 = ld_dep2(A.u + size_t(g) * 2), v2 = ld_dep2(A.v + size_t(g) * 2);
+    const float2 u2 = ld_l22(A.u + size_t(g) * 2), v2 = ld_l22(A.v + size_t(g) * 2);
     const float2 m2 = reinterpret_cast<const float2 *>(A.minv)[g];
     P.u[0] = u2.x; P.u[NC - 1] = u2.y; P.v[0] = v2.x; P.v[NC - 1] = v2.y; P.mi[0] = m2.x; P.mi[NC - 1] = m2.y;
   } else {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const size_t i = size_t(g) * NC + c;
-      P.u[c] = ld_dep(A.u + i); P.v[c] = ld_dep(A.v + i); P.mi[c] = A.minv[i];
+      P.u[c] = ld_l2(A.u + i); P.v[c] = ld_l2(A.v + i); P.mi[c] = A.minv[i];
     }
   }
   return P;
@@ -899,7 +946,7 @@ __device__ __forceinline__ bool update_point_post(const UpdateArgs &A, int g, Po
 #pragma unroll
   for (int c = 0; c < NC; ++c) a[c] = __fmul_rn(acc[c], P.mi[c]);
   if (A.rec) {
-    const size_t off = size_t(*A.step - A.rec->k0) * A.rec->stride;
+    const size_t off = size_t(A.rec_chain ? A.rec->i : *A.step - A.rec->k0) * A.rec->stride;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       A.rec->u[off + size_t(g) * NC + c] = P.u[c];

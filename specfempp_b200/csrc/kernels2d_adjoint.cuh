@@ -50,7 +50,7 @@
 // include/kokkos_kernels/frechet_kernels.hpp:37-49, compute_coupling.tpp:21-115).
 #pragma once
 
-#include "kernels2d_batched.cuh"
+#include "kernels2d_row.cuh"
 
 namespace sfg {
 namespace dev {
@@ -91,7 +91,9 @@ __global__ void __launch_bounds__(NP * E) k_adj_elem(AdjArgs A) {
   const float xix = __ldg(A.xix + p), xiz = __ldg(A.xiz + p), gax = __ldg(A.gax + p),
               gaz = __ldg(A.gaz + p), jac = __ldg(A.jac + p);
   const float c0 = __ldg(A.prop0 + p), mu = __ldg(A.prop1 + p);
-  const float2 m2 = act ? reinterpret_cast<const float2 *>(A.mu)[g] : make_float2(0.f, 0.f);
+  pdl_wait();
+  pdl_release();
+  const float2 m2 = act ? ld_dep2(A.mu + size_t(g) * 2) : make_float2(0.f, 0.f);
   const float2 u2 = act ? reinterpret_cast<const float2 *>(A.uf)[g] : make_float2(0.f, 0.f);
   const int rh = act ? __ldg(A.ad_head + e) : -1;
   sm_[0][le][q] = m2.x; sm_[1][le][q] = m2.y;
@@ -159,126 +161,6 @@ __global__ void __launch_bounds__(NP * E) k_adj_elem(AdjArgs A) {
   reinterpret_cast<float2 *>(A.seg)[p] = sg;
 }
 
-// Row form of k_adj_elem: one thread per element row (five points) of E
-// elements; the xi-direction contractions of both fields and of the
-// divergence on the row in registers (warp-uniform coefficients, the two
-// components paired in FFMA2, which rounds each lane as fmaf), the
-// gamma-direction ones from shared-memory columns.  Per point the
-// operations and their order are those of k_adj_elem (same bits).
-template <int E>
-__global__ void __launch_bounds__(NG * E, 4) k_adj_elem_row(AdjArgs A) {
-  __shared__ float2 sm2[E][NP], su2[E][NP], sF1[E][NP];
-  const int tid = threadIdx.x;
-  const int le = tid / NG, iz = tid - le * NG;
-  const int e = blockIdx.x * E + le;
-  const bool act = e < A.nspec;
-  const size_t pe = size_t(act ? e : 0) * NP + iz * NG;
-  int g[NG], sl[NG];
-  float2 mr[NG], ur[NG];
-#pragma unroll
-  for (int ix = 0; ix < NG; ++ix) g[ix] = act ? __ldg(A.ibool + pe + ix) : 0;
-#pragma unroll
-  for (int ix = 0; ix < NG; ++ix) sl[ix] = __ldg(A.pslot + pe + ix);
-#pragma unroll
-  for (int ix = 0; ix < NG; ++ix) {
-    mr[ix] = act ? reinterpret_cast<const float2 *>(A.mu)[g[ix]] : make_float2(0.f, 0.f);
-    ur[ix] = act ? reinterpret_cast<const float2 *>(A.uf)[g[ix]] : make_float2(0.f, 0.f);
-    sm2[le][iz * NG + ix] = mr[ix];
-    su2[le][iz * NG + ix] = ur[ix];
-  }
-  const int rh = act ? __ldg(A.ad_head + e) : -1;
-  // the row's Jacobian and material words, requested with the gathers
-  float gxix[NG], gxiz[NG], ggax[NG], ggaz[NG], gjac[NG], gc0[NG], gmu[NG];
-#pragma unroll
-  for (int ix = 0; ix < NG; ++ix) {
-    gxix[ix] = __ldg(A.xix + pe + ix); gxiz[ix] = __ldg(A.xiz + pe + ix);
-    ggax[ix] = __ldg(A.gax + pe + ix); ggaz[ix] = __ldg(A.gaz + pe + ix);
-    gjac[ix] = __ldg(A.jac + pe + ix); gc0[ix] = __ldg(A.prop0 + pe + ix); gmu[ix] = __ldg(A.prop1 + pe + ix);
-  }
-  float hz[NG];
-  ld_row5(t_rows[iz], hz);
-  __syncthreads();
-  // xi derivatives of both fields, both components paired, in place
-  {
-    float2 dm[NG], du[NG];
-#pragma unroll
-    for (int ix = 0; ix < NG; ++ix) {
-      float2 a = make_float2(0.f, 0.f), b = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int l = 0; l < NG; ++l) {
-        a = fma2(f2(c_hp[ix * NG + l]), mr[l], a);
-        b = fma2(f2(c_hp[ix * NG + l]), ur[l], b);
-      }
-      dm[ix] = a;
-      du[ix] = b;
-    }
-#pragma unroll
-    for (int ix = 0; ix < NG; ++ix) { mr[ix] = dm[ix]; ur[ix] = du[ix]; }
-  }
-  const float wiz = ld_w(iz);
-#pragma unroll
-  for (int ix = 0; ix < NG; ++ix) {
-    const size_t p = pe + ix;
-    const float xix = gxix[ix], xiz = gxiz[ix], gax = ggax[ix], gaz = ggaz[ix], jac = gjac[ix];
-    const float c0 = gc0[ix], mu = gmu[ix];
-    float2 gm = make_float2(0.f, 0.f), gu = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int l = 0; l < NG; ++l) {
-      gm = fma2(f2(hz[l]), sm2[le][l * NG + ix], gm);
-      gu = fma2(f2(hz[l]), su2[le][l * NG + ix], gu);
-    }
-    // dm[c][0] = mr[ix].c (xi), dm[c][1] = gm.c (gamma)
-    const float mxx = xix * mr[ix].x + gax * gm.x, mxz = xiz * mr[ix].x + gaz * gm.x;
-    const float mzx = xix * mr[ix].y + gax * gm.y, mzz = xiz * mr[ix].y + gaz * gm.y;
-    const float uxx = xix * ur[ix].x + gax * gu.x, uxz = xiz * ur[ix].x + gaz * gu.x;
-    const float uzx = xix * ur[ix].y + gax * gu.y, uzz = xiz * ur[ix].y + gaz * gu.y;
-    const float lam = c0 - 2.f * mu;
-    const float sxx = c0 * mxx + lam * mzz;
-    const float szz = c0 * mzz + lam * mxx;
-    const float sxz = mu * (mxz + mzx);
-    mr[ix] = make_float2(jac * (sxx * xix + sxz * xiz), jac * (sxz * xix + szz * xiz));   // F0
-    sF1[le][iz * NG + ix] = make_float2(jac * (sxx * gax + sxz * gaz), jac * (sxz * gax + szz * gaz));
-    if (act) {
-      // gradient terms of this step, summed over the segment
-      const float W = c_w[ix] * wiz * jac;
-      const float divm = mxx + mzz, divu = uxx + uzz;
-      const float tk = -W * (divm * divu);
-      const float tm = -W * ((4.f / 3.f) * (mxx * uxx + mzz * uzz) - (2.f / 3.f) * (mxx * uzz + mzz * uxx) +
-                             (mxz + mzx) * (uxz + uzx));
-      float2 sg = reinterpret_cast<float2 *>(A.seg)[p];
-      sg.x += tk;
-      sg.y += tm;
-      reinterpret_cast<float2 *>(A.seg)[p] = sg;
-    }
-  }
-  float wz[NG];
-  ld_row5(t_rows[5 + iz], wz);
-  __syncthreads();
-  if (!act) return;
-#pragma unroll
-  for (int ix = 0; ix < NG; ++ix) {
-    const int q = iz * NG + ix;
-    float2 t1 = make_float2(0.f, 0.f), t2 = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int l = 0; l < NG; ++l) {
-      t1 = fma2(mr[l], f2(c_hpw[l * NG + ix]), t1);
-      t2 = fma2(sF1[le][l * NG + ix], f2(wz[l]), t2);
-    }
-    float r0 = -(wiz * t1.x + c_w[ix] * t2.x);
-    float r1 = -(wiz * t1.y + c_w[ix] * t2.y);
-    // receivers of this element inject R^T g (the adjoint sources)
-    if (rh >= 0) {
-      const float *g_k = A.gtab + size_t(*A.seg_k0 + A.slot) * A.nrec * 2;
-      for (int k = rh; k >= 0; k = A.ad_next[k]) {
-        const float h = A.ad_h[size_t(k) * NP + q];
-        r0 += g_k[2 * k] * h;
-        r1 += g_k[2 * k + 1] * h;
-      }
-    }
-    reinterpret_cast<float2 *>(A.r)[sl[ix]] = make_float2(r0, r1);
-  }
-}
-
 // SH reverse element step (one component): -K mu with sigma = mu grad,
 // adjoint sources R^T g (first seismogram component, BXY), and the mu term.
 template <int E>
@@ -296,7 +178,9 @@ __global__ void __launch_bounds__(NP * E) k_adj_elem_sh(AdjArgs A) {
   const float xix = __ldg(A.xix + p), xiz = __ldg(A.xiz + p), gax = __ldg(A.gax + p),
               gaz = __ldg(A.gaz + p), jac = __ldg(A.jac + p);
   const float mu = __ldg(A.prop1 + p);
-  sm_[le][q] = act ? A.mu[g] : 0.f;
+  pdl_wait();
+  pdl_release();
+  sm_[le][q] = act ? ld_dep(A.mu + g) : 0.f;
   su_[le][q] = act ? A.uf[g] : 0.f;
   const int rh = act ? __ldg(A.ad_head + e) : -1;
   __syncthreads();
@@ -350,7 +234,9 @@ __global__ void __launch_bounds__(NP * E) k_adj_elem_ac(AdjArgs A) {
   const float xix = __ldg(A.xix + p), xiz = __ldg(A.xiz + p), gax = __ldg(A.gax + p),
               gaz = __ldg(A.gaz + p), jac = __ldg(A.jac + p);
   const float rhoinv = __ldg(A.prop0 + p);
-  float m = act ? A.mu[g] : 0.f;
+  pdl_wait();
+  pdl_release();
+  float m = act ? ld_dep(A.mu + g) : 0.f;
   const int bs = act ? __ldg(A.bc_slot + e) : -1;
   if (bs >= 0) m *= A.bc_keep[size_t(bs) * NP + q];
   sm_[le][q] = m;
@@ -392,6 +278,8 @@ __global__ void __launch_bounds__(128) k_adj_psrc(float *__restrict__ mu, const 
                                                   const int *__restrict__ rec, const float *__restrict__ hw,
                                                   const float *__restrict__ gtab, const int *__restrict__ seg_k0,
                                                   int slot, int nrec, int n) {
+  pdl_wait();
+  pdl_release();
   const int k = *seg_k0 + slot;
   if (k < 0) return;
   const float *g_k = gtab + size_t(k) * nrec * 2;
@@ -414,12 +302,14 @@ __global__ void __launch_bounds__(128) k_adj_srcterm(float *__restrict__ acc, co
                                                      const float *__restrict__ stf, const int *__restrict__ seg_k0,
                                                      int slot, int nsrc, int nstep, const int *__restrict__ src_id,
                                                      int stf_cols) {
+  pdl_wait();
+  pdl_release();
   const int k = *seg_k0 + slot;
   if (k >= nstep) return;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nsrc * NP; t += gridDim.x * blockDim.x) {
     const int s = t / NP, q = t - s * NP;
     const int g = ibool[size_t(src_ce[s]) * NP + q];
-    acc[t] += mu[g] * stf[size_t(k) * stf_cols + (src_id ? src_id[s] : s)];
+    acc[t] += ld_dep(mu + g) * stf[size_t(k) * stf_cols + (src_id ? src_id[s] : s)];
   }
 }
 
@@ -451,24 +341,26 @@ __global__ void __launch_bounds__(256) k_adj_post(float *__restrict__ lu, float 
                                                   const float *__restrict__ minv,
                                                   const float *__restrict__ r,
                                                   const int *__restrict__ inv_start, int npts, float dt,
-                                                  float dt2, float dtsq2, AdjCoupling cp = AdjCoupling{}) {
+                                                  float dt2, float dtsq2, AdjCoupling cp) {
+  pdl_wait();
+  pdl_release();
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < npts; g += gridDim.x * blockDim.x) {
     float s[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) s[c] = 0.f;
     for (int k = inv_start[g]; k < inv_start[g + 1]; ++k) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) s[c] = s[c] + r[size_t(k) * NC + c];
+      for (int c = 0; c < NC; ++c) s[c] = s[c] + ld_dep(r + size_t(k) * NC + c);
     }
     float cpa = 0.f;
     if (CPL && g < cp.niface) {
       const int o2 = cp.other[g];
       if (NC == 2) {
-        const float m = cp.omu[o2];
+        const float m = ld_dep(cp.omu + o2);
         s[0] = s[0] + cp.nx[g] * m;
         s[NC - 1] = s[NC - 1] + cp.nz[g] * m;
       } else {
-        cpa = cp.nx[g] * cp.omu[2 * size_t(o2)] + cp.nz[g] * cp.omu[2 * size_t(o2) + 1];
+        cpa = cp.nx[g] * ld_dep(cp.omu + 2 * size_t(o2)) + cp.nz[g] * ld_dep(cp.omu + 2 * size_t(o2) + 1);
       }
     }
     const size_t o = size_t(g) * NC;
@@ -525,7 +417,7 @@ __device__ __forceinline__ void adj_stacey_grad(const int *__restrict__ lb_g, co
     // SH: C = wq j1 rvs, only A2 = mu v~ and A4 = mu a'
     for (int i = first; i < n; i += stride) {
       const int g = lb_g[i];
-      const float m = mu[g];
+      const float m = ld_dep(mu + g);
       float4 t = reinterpret_cast<float4 *>(acc)[i];
       t.y += geo[i].x * (m * vst[lb_j[i]]);     // x: 1, or the acoustic free-surface mask
       t.w += m * af[g];
@@ -535,7 +427,7 @@ __device__ __forceinline__ void adj_stacey_grad(const int *__restrict__ lb_g, co
     for (int i = first; i < n; i += stride) {
       const int g = lb_g[i];
       const float4 q = geo[i];
-      const float2 m = reinterpret_cast<const float2 *>(mu)[g];
+      const float2 m = ld_dep2(mu + size_t(g) * 2);
       const float2 v = reinterpret_cast<const float2 *>(vst)[lb_j[i]];
       const float2 a = reinterpret_cast<const float2 *>(af)[g];
       const float inv = 1.0f / (q.z * q.z);
@@ -567,23 +459,181 @@ struct AdjStaceyArgs {
   int nb_grad;
 };
 
+// Block b of nb.
 template <int NC>
-__global__ void __launch_bounds__(256) k_adj_stacey(AdjStaceyArgs S) {
-  if (int(blockIdx.x) < S.nb_grad) {
+__device__ __forceinline__ void adj_stacey(const AdjStaceyArgs &S, int b, int nb) {
+  if (b < S.nb_grad) {
     adj_stacey_grad<NC>(S.lb_g, S.lb_j, S.geo, S.mu, S.vst, S.af, S.acc, S.nlb,
-                    blockIdx.x * blockDim.x + threadIdx.x, S.nb_grad * blockDim.x);
+                    b * blockDim.x + threadIdx.x, S.nb_grad * blockDim.x);
     return;
   }
-  const int stride = (gridDim.x - S.nb_grad) * blockDim.x;
-  for (int j = (blockIdx.x - S.nb_grad) * blockDim.x + threadIdx.x; j < S.nst; j += stride) {
+  const int stride = (nb - S.nb_grad) * blockDim.x;
+  for (int j = (b - S.nb_grad) * blockDim.x + threadIdx.x; j < S.nst; j += stride) {
     const int g = S.pt[j];
     if (NC == 1) {
-      S.lv[g] -= S.cm[3 * j] * S.mu[g];    // SH: C scalar in the xx slot
+      S.lv[g] -= S.cm[3 * j] * ld_dep(S.mu + g);    // SH: C scalar in the xx slot
       continue;
     }
-    const float mx = S.mu[2 * g], mz = S.mu[2 * g + 1];
+    const float2 m2 = ld_dep2(S.mu + size_t(g) * 2);
+    const float mx = m2.x, mz = m2.y;
     S.lv[2 * g] -= S.cm[3 * j] * mx + S.cm[3 * j + 1] * mz;
     S.lv[2 * g + 1] -= S.cm[3 * j + 1] * mx + S.cm[3 * j + 2] * mz;
+  }
+}
+
+template <int NC>
+__global__ void __launch_bounds__(256) k_adj_stacey(AdjStaceyArgs S) {
+  pdl_wait();
+  pdl_release();
+  adj_stacey<NC>(S, blockIdx.x, gridDim.x);
+}
+
+// Row form of k_adj_elem with the step's Stacey part in its first blocks
+// (they read mu and touch lv and the impedance sums, the element blocks mu, r
+// and the point sums: nothing in common but mu).  One thread per element row
+// (five points) of E elements: the xi-direction contractions of both fields
+// and of the divergence on the row in registers (the two components paired in
+// FFMA2, which rounds each lane as fmaf), the gamma-direction ones from
+// shared-memory columns; points gathered, summed and scattered by consecutive
+// threads, and the mesh's one-value words from the element's record, as in
+// k_stiffness_row (GEO, MAT).  Per point the operations and their order are
+// those of k_adj_elem (same bits).
+template <int E, int GEO, int MAT>
+__global__ void __launch_bounds__(NG * E, 4) k_adj_elem_row(AdjArgs A, MedArgs W, AdjStaceyArgs S, int stacey_blocks) {
+  constexpr int T = NG * E;
+  __shared__ __align__(16) float smem[NP * E * (6 + (GEO ? 0 : 5) + (MAT ? 0 : 2))];
+  const int tid = threadIdx.x;
+  const int b = int(blockIdx.x) - stacey_blocks;
+  if (b < 0) {
+    pdl_wait();
+    pdl_release();
+    adj_stacey<2>(S, blockIdx.x, stacey_blocks);
+    return;
+  }
+  float2 *smb = reinterpret_cast<float2 *>(smem), *sub = smb + NP * E, *sFb = sub + NP * E;   // mu, u~, F1
+  float *sg = smem + 6 * NP * E, *sm = sg + (GEO ? 0 : 5 * NP * E);
+  const int le = tid / NG, iz = tid - le * NG;
+  const int e = b * E + le;
+  const bool act = e < A.nspec;
+  const float2 *sm2 = smb + le * NP, *su2 = sub + le * NP;
+  float2 *sF1 = sFb + le * NP;
+  const size_t p0 = size_t(b) * E * NP, pend = size_t(A.nspec) * NP, rec = size_t(act ? e : 0) * 8;
+  RowGeo<E, GEO> G;
+  RowMat<E, MAT> M;
+  G.stage(W, p0, sg);
+  M.stage(W, p0, sm);
+  int g[NG], sl[NG];
+#pragma unroll
+  for (int k = 0; k < NG; ++k) {
+    const size_t p = p0 + tid + k * T;
+    g[k] = p < pend ? __ldg(A.ibool + p) : -1;
+    sl[k] = p < pend ? __ldg(A.pslot + p) : 0;
+  }
+  G.load(W, rec, sg, tid * NG);
+  M.load(W, rec, sm, tid * NG);
+  // the recorded u~ of the step is not written by the sweep
+#pragma unroll
+  for (int k = 0; k < NG; ++k)
+    sub[tid + k * T] = g[k] >= 0 ? reinterpret_cast<const float2 *>(A.uf)[g[k]] : make_float2(0.f, 0.f);
+  const int rh = act ? __ldg(A.ad_head + e) : -1;
+  float hz[NG];
+  ld_row5(t_rows[iz], hz);
+  const float wiz = ld_w(iz);
+  pdl_wait();
+  pdl_release();
+  {
+    float2 t[NG];
+#pragma unroll
+    for (int k = 0; k < NG; ++k) t[k] = g[k] >= 0 ? ld_dep2(A.mu + size_t(g[k]) * 2) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < NG; ++k) smb[tid + k * T] = t[k];
+  }
+  if (GEO == 0 || MAT == 0) cp_async_wait();
+  __syncthreads();
+  // xi derivatives of both fields, both components paired
+  float2 mr[NG], ur[NG];
+  {
+    float2 x[NG], y[NG];
+#pragma unroll
+    for (int l = 0; l < NG; ++l) { x[l] = sm2[iz * NG + l]; y[l] = su2[iz * NG + l]; }
+#pragma unroll
+    for (int ix = 0; ix < NG; ++ix) {
+      float2 p = make_float2(0.f, 0.f), q = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int l = 0; l < NG; ++l) {
+        p = fma2(f2(c_hp[ix * NG + l]), x[l], p);
+        q = fma2(f2(c_hp[ix * NG + l]), y[l], q);
+      }
+      mr[ix] = p;
+      ur[ix] = q;
+    }
+  }
+#pragma unroll
+  for (int ix = 0; ix < NG; ++ix) {
+    float2 gm = make_float2(0.f, 0.f), gu = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int l = 0; l < NG; ++l) {
+      gm = fma2(f2(hz[l]), sm2[l * NG + ix], gm);
+      gu = fma2(f2(hz[l]), su2[l * NG + ix], gu);
+    }
+    const auto P = G.at(ix);
+    const float c0 = M.c0(ix), mu = M.mu(ix);
+    const float mxx = P.ddx(mr[ix].x, gm.x), mxz = P.ddz(mr[ix].x, gm.x);
+    const float mzx = P.ddx(mr[ix].y, gm.y), mzz = P.ddz(mr[ix].y, gm.y);
+    const float uxx = P.ddx(ur[ix].x, gu.x), uxz = P.ddz(ur[ix].x, gu.x);
+    const float uzx = P.ddx(ur[ix].y, gu.y), uzz = P.ddz(ur[ix].y, gu.y);
+    const float lam = c0 - 2.f * mu;
+    const float sxx = c0 * mxx + lam * mzz;
+    const float szz = c0 * mzz + lam * mxx;
+    const float sxz = mu * (mxz + mzx);
+    mr[ix] = make_float2(P.f0(sxx, sxz), P.f0(sxz, szz));   // F0
+    sF1[iz * NG + ix] = make_float2(P.f1(sxx, sxz), P.f1(sxz, szz));
+    // gradient terms of this step
+    const float Wq = c_w[ix] * wiz * G.j(ix);
+    const float divm = mxx + mzz, divu = uxx + uzz;
+    const float tk = -Wq * (divm * divu);
+    const float tm = -Wq * ((4.f / 3.f) * (mxx * uxx + mzz * uzz) - (2.f / 3.f) * (mxx * uzz + mzz * uxx) +
+                            (mxz + mzx) * (uxz + uzx));
+    ur[ix] = make_float2(tk, tm);
+  }
+  float wz[NG];
+  ld_row5(t_rows[5 + iz], wz);
+  __syncthreads();
+#pragma unroll
+  for (int ix = 0; ix < NG; ++ix) {
+    const int q = iz * NG + ix;
+    float2 t1 = make_float2(0.f, 0.f), t2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int l = 0; l < NG; ++l) {
+      t1 = fma2(mr[l], f2(c_hpw[l * NG + ix]), t1);
+      t2 = fma2(sF1[l * NG + ix], f2(wz[l]), t2);
+    }
+    float r0 = -(wiz * t1.x + c_w[ix] * t2.x);
+    float r1 = -(wiz * t1.y + c_w[ix] * t2.y);
+    // receivers of this element inject R^T g (the adjoint sources)
+    if (rh >= 0) {
+      const float *g_k = A.gtab + size_t(*A.seg_k0 + A.slot) * A.nrec * 2;
+      for (int k = rh; k >= 0; k = A.ad_next[k]) {
+        const float h = A.ad_h[size_t(k) * NP + q];
+        r0 += g_k[2 * k] * h;
+        r1 += g_k[2 * k + 1] * h;
+      }
+    }
+    // both fields have been read by all: their places take the results
+    smb[le * NP + q] = make_float2(r0, r1);
+    sub[le * NP + q] = ur[ix];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NG; ++k) {
+    if (g[k] < 0) continue;
+    const int i = tid + k * T;
+    reinterpret_cast<float2 *>(A.r)[sl[k]] = smb[i];
+    float2 *seg = reinterpret_cast<float2 *>(A.seg) + p0 + i;
+    float2 t = *seg;
+    t.x += sub[i].x;
+    t.y += sub[i].y;
+    *seg = t;
   }
 }
 

@@ -432,15 +432,15 @@ __host__ __device__ constexpr int row_min_blocks() {
   return 65536 / (threads * regs);
 }
 
-// The first rec_blocks blocks take receivers, the next el.nblocks elastic
+// The first blocks take receivers and the recording of a step, the next el.nblocks elastic
 // elements (EK 0 P-SV, 1 SH, 4 poroelastic; 5 none), the others acoustic ones
 // (EK 0 and 5).
 template <int E, int EK, int GEO, int MAT>
 __global__ void __launch_bounds__(NG * E, row_min_blocks<E, EK, GEO, MAT>()) k_stiffness_row(StiffArgs S) {
   __shared__ __align__(16) float smem[row_smem<E, EK, GEO, MAT>()];
-  const int b = int(blockIdx.x) - S.rec_blocks;
+  const int b = int(blockIdx.x) - S.rec_blocks - S.save_blocks;
   if (b < 0) {
-    receiver_blocks(S.rec_ac, S.rec_el, S.nrec_ac, S.nrec_el, smem);
+    leading_block(S, smem);
   } else if (EK != 5 && b < S.el.nblocks) {
     if (EK == 1) scalar_rows<E, true, GEO, MAT>(S, S.el, S.el.e0 + b * E, smem);
     else pair_rows<E, EK == 4 ? 4 : 0, GEO, MAT>(S, S.el, S.el.e0 + b * E, smem);

@@ -423,6 +423,12 @@ void early_receivers(const sfg_handle *h, sfg::dev::StiffArgs &S, int threads, b
   S.rec_el = h->d_rec_args + 1;
   const int nw = threads / 32;
   S.rec_blocks = (S.nrec_ac + S.nrec_el + nw - 1) / nw;
+  if (h->recording && chained(h)) {
+    // a recorded step: up to 8 blocks store v~ at the Stacey points
+    S.save_el = h->adj.d_rec;
+    S.save_ac = h->adj_coupled ? h->adj2.d_rec : nullptr;
+    S.save_blocks = std::max(1, std::min(8, (std::max(h->adj.nst, h->adj2.nst) * 2 + threads - 1) / threads));
+  }
 }
 
 template <int E, int EK>
@@ -451,7 +457,7 @@ void launch_stiffness_E(sfg_handle *h, const DevMedium &el, const DevMedium &ac,
     S.el.e0 = 0; S.el.e1 = el.nspec; S.el.nblocks = (el.nspec + E - 1) / E;
     S.ac.e0 = 0; S.ac.e1 = ac.nspec; S.ac.nblocks = (ac.nspec + E - 1) / E;
     early_receivers(h, S, sfg::dev::NP * E, h->early_now[0], h->early_now[1]);
-    const int grid = S.el.nblocks + S.ac.nblocks + S.rec_blocks;
+    const int grid = S.el.nblocks + S.ac.nblocks + S.rec_blocks + S.save_blocks;
     if (grid > 0) launch_pdl(sfg::dev::k_stiffness<E, EK, true>, grid, sfg::dev::NP * E, 0, s, S);
     return;
   }
@@ -651,7 +657,7 @@ void launch_stiffness_row(sfg_handle *h, const DevMedium &el, const DevMedium &a
   S.el.e0 = 0; S.el.e1 = el.nspec; S.el.nblocks = (el.nspec + E - 1) / E;
   S.ac.e0 = 0; S.ac.e1 = ac.nspec; S.ac.nblocks = (ac.nspec + E - 1) / E;
   early_receivers(h, S, sfg::dev::NG * E, h->early_now[0], h->early_now[1]);
-  const int grid = S.el.nblocks + S.ac.nblocks + S.rec_blocks;
+  const int grid = S.el.nblocks + S.ac.nblocks + S.rec_blocks + S.save_blocks;
   if (grid == 0) return;
   if (!S.el.erec && !S.ac.erec) throw std::runtime_error("row-form element kernel: element records missing on the device");
   const int geo = row_straight(h) ? 1 : 0, mat = row_matconst(h) ? 1 : 0;
@@ -723,7 +729,8 @@ sfg::dev::UpdateArgs update_args(sfg_handle *h, const DevMedium &D, const DevMed
   }
   U.flag = h->d_flag;
   U.step = h->d_step;
-  U.advance = advance && !h->recording ? 1 : 0;
+  U.advance = advance && (!h->recording || chained(h)) ? 1 : 0;
+  U.rec_chain = chained(h) ? 1 : 0;
   if (h->recording) U.rec = (h->adj_coupled && medium == SFG_MEDIUM_ACOUSTIC) ? h->adj2.d_rec : h->adj.d_rec;
   return U;
 }
@@ -1376,7 +1383,7 @@ void enqueue_step(sfg_handle *h, cudaStream_t s, bool predict) {
     return;
   }
   const bool has_el = h->el.nspec > 0, has_ac = h->ac.nspec > 0;
-  if (h->recording) {
+  if (h->recording && !chained(h)) {
     const DevMedium &R = h->el.nspec ? h->el : h->ac;
     if (R.ncomp == 1) sfg::dev::k_record_begin<1><<<1, 512, 0, s>>>(h->adj.d_rec, R.v, h->d_step);
     else sfg::dev::k_record_begin<2><<<1, 512, 0, s>>>(h->adj.d_rec, R.v, h->d_step);
@@ -1446,7 +1453,7 @@ int kernels_per_step(const sfg_handle *h) {
 }
 
 bool fused_update(const sfg_handle *h) {
-  if (!h->fuse_ok || h->variant < 3 || h->recording) return false;
+  if (!h->fuse_ok || h->variant < 3 || (h->recording && !chained(h))) return false;
   const sfg::Assembly2D &a = h->asmb;
   if (h->el.nrec == 0) return true;
   for (int t : a.types)
@@ -1465,13 +1472,15 @@ cudaGraphExec_t capture(sfg_handle *h, int nsteps, bool last_predicts) {
   return ex;
 }
 
-// Capture the step graphs (again); the streamed and the recording steps'
-// graphs are captured when they are next used.
+// Capture the step graphs (again); the streamed, the recording and the reverse
+// steps' graphs are captured when they are next used.
 void recapture(sfg_handle *h) {
   SFG_CUDA(cudaStreamSynchronize(h->stream));
   for (cudaGraphExec_t *g : {&h->graph_k, &h->graph_1, &h->graph_e, &h->graph_io, &h->adj.graph_r1, &h->adj.graph_re,
                              &h->adj.graph_rseg})
     if (*g) { cudaGraphExecDestroy(*g); *g = nullptr; }
+  for (cudaGraphExec_t &g : h->adj.graph_rev)
+    if (g) { cudaGraphExecDestroy(g); g = nullptr; }
   h->graph_k = capture(h, h->graph_steps, true);
   h->graph_1 = capture(h, 1, true);
   h->graph_e = capture(h, 1, false);
@@ -2408,8 +2417,8 @@ int sfg_set_model2d(sfg_handle *h, const float *rho, const float *kappa, const f
         put(D.minv, M.minv);
         put(D.erec, M.row.erec);
       }
-      // the step graphs hold the element kernel of the old model's class
-      if (row_matconst(h) != mat0 && (h->variant == 6 || (h->asmb.nshots > 1 && h->variant == 4))) recapture(h);
+      // the step graphs hold the element kernels of the old model's class
+      if (row_matconst(h) != mat0) recapture(h);
       refresh_tile_records(h);
       if (h->adj.st_c && !h->asmb.el.stacey_c.empty())
         SFG_CUDA(cudaMemcpy(h->adj.st_c, h->asmb.el.stacey_c.data(), h->asmb.el.stacey_c.size() * sizeof(float),
@@ -2606,8 +2615,8 @@ void adj_medium_init(sfg_handle *h, AdjointState &A, const DevMedium &D, const s
   A.d_rec = dalloc<sfg::dev::SegRecord>(1);
 }
 
-void adj_write_record(AdjointState &A) {
-  sfg::dev::SegRecord rec{A.seg_u, A.seg_a, A.stride, 0, A.seg_v, A.vstride, A.st_pt, A.nst, 0};
+void adj_write_record(AdjointState &A, const DevMedium &D) {
+  sfg::dev::SegRecord rec{A.seg_u, A.seg_a, A.stride, 0, A.seg_v, A.vstride, A.st_pt, A.nst, D.ncomp, D.v, 0};
   SFG_CUDA(cudaMemcpy(A.d_rec, &rec, sizeof(rec), cudaMemcpyHostToDevice));
 }
 
@@ -2661,8 +2670,8 @@ void adjoint_alloc(sfg_handle *h, int nstep, int interval) {
     SFG_CUDA(cudaStreamCreateWithFlags(&A.rstream, cudaStreamNonBlocking));
   }
   if (cpl && !A2.lu) adj_medium_init(h, A2, h->ac, h->asmb.ac, SFG_MEDIUM_ACOUSTIC);
-  adj_write_record(A);
-  if (cpl) adj_write_record(A2);
+  adj_write_record(A, D);
+  if (cpl) adj_write_record(A2, h->ac);
   if (!A.graph_r1) {
     // one recording step with the next predictor fused, and one ending on
     // the corrector (the segment's last step)
@@ -2763,14 +2772,26 @@ void reverse_segment_E(sfg_handle *h, int b, int n, bool last, cudaStream_t rs) 
   const size_t ob = size_t(b) * A.interval;
   auto psrc = [&](AdjointState &X, const DevMedium &M, int slot) {
     if (X.nps)
-      sfg::dev::k_adj_psrc<<<std::min(grid_for(X.nps), 64), 128, 0, rs>>>(
+      launch_pdl(sfg::dev::k_adj_psrc, std::min(grid_for(X.nps), 64), 128, 0, rs,
           X.mu, M.minv, X.ps_pt, X.ps_start, X.ps_rec, X.ps_h, A.gtab, A.d_k0, slot, h->asmb.nrec, X.nps);
   };
   auto srcterm = [&](AdjointState &X, const DevMedium &M, int slot) {
     if (X.nsrc_t)
-      sfg::dev::k_adj_srcterm<<<(X.nsrc_t * sfg::NPTS + 127) / 128, 128, 0, rs>>>(
+      launch_pdl(sfg::dev::k_adj_srcterm, (X.nsrc_t * sfg::NPTS + 127) / 128, 128, 0, rs,
           X.seg + X.off_src(), X.mu, M.ibool, X.src_ce, h->d_stf, A.d_k0, slot, X.nsrc_t, h->asmb.nstep,
           X.src_id, h->asmb.nsrc);
+  };
+  // the row form, with the step's Stacey part in its first blocks
+  auto row_elem = [&](bool stacey) {
+    const int sb = stacey ? St.nb_grad + grid_for(A.nst) : 0;
+    const bool geo = h->asmb.el.row.straight, mat = h->asmb.el.row.matconst;
+    auto go = [&](auto kern) {
+      launch_pdl(kern, (D.nspec + 31) / 32 + sb, sfg::dev::NG * 32, 0, rs, J, med_args(D), St, sb);
+    };
+    if (geo && mat) go(sfg::dev::k_adj_elem_row<32, 1, 1>);
+    else if (geo) go(sfg::dev::k_adj_elem_row<32, 1, 0>);
+    else if (mat) go(sfg::dev::k_adj_elem_row<32, 0, 1>);
+    else go(sfg::dev::k_adj_elem_row<32, 0, 0>);
   };
   if (h->adj_coupled) {
     // coupled P-SV + acoustic step in reverse: both media's Stacey and
@@ -2790,25 +2811,25 @@ void reverse_segment_E(sfg_handle *h, int b, int n, bool last, cudaStream_t rs) 
       if (A.nst) {
         St.vst = A.seg_v + sl * A.vstride;
         St.af = A.seg_a + sl * A.stride;
-        sfg::dev::k_adj_stacey<2><<<St.nb_grad + grid_for(A.nst), 256, 0, rs>>>(St);
+        if (!ROW) launch_pdl(sfg::dev::k_adj_stacey<2>, St.nb_grad + grid_for(A.nst), 256, 0, rs, St);
       }
       if (C.nst) {
         Sa.vst = C.seg_v + sl * C.vstride;
         Sa.af = C.seg_a + sl * C.stride;
-        sfg::dev::k_adj_stacey<1><<<Sa.nb_grad + grid_for(C.nst), 256, 0, rs>>>(Sa);
+        launch_pdl(sfg::dev::k_adj_stacey<1>, Sa.nb_grad + grid_for(C.nst), 256, 0, rs, Sa);
       }
       J.uf = A.seg_u + sl * A.stride;
       J.slot = i;
-      if (ROW) sfg::dev::k_adj_elem_row<32><<<(D.nspec + 31) / 32, sfg::dev::NG * 32, 0, rs>>>(J);
-      else sfg::dev::k_adj_elem<E><<<eblocks, sfg::dev::NP * E, 0, rs>>>(J);
+      if (ROW) row_elem(A.nst > 0);
+      else launch_pdl(sfg::dev::k_adj_elem<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
       Ja.uf = C.seg_u + sl * C.stride;
       Ja.slot = i;
-      sfg::dev::k_adj_elem_ac<E><<<ablocks, sfg::dev::NP * E, 0, rs>>>(Ja);
+      launch_pdl(sfg::dev::k_adj_elem_ac<E>, ablocks, sfg::dev::NP * E, 0, rs, Ja);
       srcterm(C, Ac, i);
-      sfg::dev::k_adj_post<2, true><<<grid_for(D.nglob), 256, 0, rs>>>(
+      launch_pdl(sfg::dev::k_adj_post<2, true>, grid_for(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
           D.nglob, dt, dt2, dtsq2, cp_el);
-      sfg::dev::k_adj_post<1, true><<<grid_for(Ac.nglob), 256, 0, rs>>>(
+      launch_pdl(sfg::dev::k_adj_post<1, true>, grid_for(Ac.nglob), 256, 0, rs,
           C.lu, C.lv, C.mu, C.seg + 2 * C.nloc, C.seg_a + sl * C.stride, Ac.minv, C.r, Ac.inv_start,
           Ac.nglob, dt, dt2, dtsq2, cp_ac);
       psrc(C, Ac, i - 1);
@@ -2821,32 +2842,34 @@ void reverse_segment_E(sfg_handle *h, int b, int n, bool last, cudaStream_t rs) 
   for (int i = n - 1; i >= 0; --i) {
     const size_t sl = ob + size_t(i);
     const bool sh = D.ncomp == 1;
-    if (A.nst && !(last && i == n - 1 && !A.pressure)) {
+    const bool stacey = A.nst && !(last && i == n - 1 && !A.pressure);
+    if (stacey) {
       St.vst = A.seg_v + sl * A.vstride;
       St.af = A.seg_a + sl * A.stride;
-      if (sh) sfg::dev::k_adj_stacey<1><<<St.nb_grad + grid_for(A.nst), 256, 0, rs>>>(St);
-      else sfg::dev::k_adj_stacey<2><<<St.nb_grad + grid_for(A.nst), 256, 0, rs>>>(St);
+      if (ROW) {}      // in the element launch
+      else if (sh) launch_pdl(sfg::dev::k_adj_stacey<1>, St.nb_grad + grid_for(A.nst), 256, 0, rs, St);
+      else launch_pdl(sfg::dev::k_adj_stacey<2>, St.nb_grad + grid_for(A.nst), 256, 0, rs, St);
     }
     J.uf = A.seg_u + sl * A.stride;
     J.slot = i;
     if (A.pressure) {
-      sfg::dev::k_adj_elem_ac<E><<<eblocks, sfg::dev::NP * E, 0, rs>>>(J);
+      launch_pdl(sfg::dev::k_adj_elem_ac<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
       srcterm(A, D, i);
-      sfg::dev::k_adj_post<1><<<grid_for(D.nglob), 256, 0, rs>>>(
+      launch_pdl(sfg::dev::k_adj_post<1, false>, grid_for(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
-          D.nglob, dt, dt2, dtsq2);
+          D.nglob, dt, dt2, dtsq2, sfg::dev::AdjCoupling{});
       psrc(A, D, i - 1);                      // mu of the previous step gets its source
     } else if (sh) {
-      sfg::dev::k_adj_elem_sh<E><<<eblocks, sfg::dev::NP * E, 0, rs>>>(J);
-      sfg::dev::k_adj_post<1><<<grid_for(D.nglob), 256, 0, rs>>>(
+      launch_pdl(sfg::dev::k_adj_elem_sh<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
+      launch_pdl(sfg::dev::k_adj_post<1, false>, grid_for(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
-          D.nglob, dt, dt2, dtsq2);
+          D.nglob, dt, dt2, dtsq2, sfg::dev::AdjCoupling{});
     } else {
-      if (ROW) sfg::dev::k_adj_elem_row<32><<<(D.nspec + 31) / 32, sfg::dev::NG * 32, 0, rs>>>(J);
-      else sfg::dev::k_adj_elem<E><<<eblocks, sfg::dev::NP * E, 0, rs>>>(J);
-      sfg::dev::k_adj_post<2><<<grid_for(D.nglob), 256, 0, rs>>>(
+      if (ROW) row_elem(stacey);
+      else launch_pdl(sfg::dev::k_adj_elem<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
+      launch_pdl(sfg::dev::k_adj_post<2, false>, grid_for(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
-          D.nglob, dt, dt2, dtsq2);
+          D.nglob, dt, dt2, dtsq2, sfg::dev::AdjCoupling{});
     }
   }
   sfg::dev::k_kahan_fold<<<grid_for(int(A.nsum())), 256, 0, rs>>>(A.sum, A.comp, A.seg, int(A.nsum()));
