@@ -130,11 +130,11 @@ typedef struct sfg_options {
                                     launch; isotropic P-SV / SH / acoustic media, or
                                     batched shots in fours on one elastic medium, others
                                     fall back to 3); with batched shots 2 is 1 and 4 is
-                                    owner-computes with the row-form element kernel (one
-                                    thread per element row and quad of shots; shots in
-                                    fours); 6 owner-computes with the row-form element
+                                    owner-computes with one thread per element and shot;
+                                    6 owner-computes with the row-form element
                                     kernel of one shot (one thread per element row;
-                                    isotropic P-SV and acoustic media, 16 or 32 elements
+                                    isotropic P-SV and acoustic media, SH and poroelastic
+                                    ones alone, 16 or 32 elements
                                     per block, others fall back to 3); with batched shots
                                     in fours and displacement receivers, 7 assembles and
                                     finishes each four-element tile's interior points in

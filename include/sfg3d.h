@@ -4,10 +4,9 @@
  * 8-node hexahedra (arbitrary control-node coordinates), isotropic elastic
  * media given per GLL point, force and moment-tensor sources, receivers, the
  * Newmark time loop captured in CUDA graphs.  Status codes and sfg_options
- * are those of sfg.h (elements_per_block fixes the element kernel's launch
- * shape: 1, 2 or 4 elements per block with one thread per element GLL point,
- * 6 or 8 with one thread per column of five points; 0 lets the autotuner
- * choose; all give the same bits; kernel_variant is ignored).
+ * are those of sfg.h (elements_per_block, 1, 2, 4, 6 or 8, fixes the layers of
+ * elements that a block of the layer kernel marches through; 0 lets the
+ * autotuner choose; all give the same bits; kernel_variant is ignored).
  *
  * It replaces, for this mesh class, the reference's dim3 forward path:
  * the assembly (core/specfem/assembly/ dim3 containers), the element kernel
@@ -53,7 +52,7 @@ typedef struct sfg_info3d {
   size_t device_bytes;
   int elements_per_block;
   int kernels_per_step;
-  int kernel_variant;           /* element-kernel form in use: 1 point form, 2 column form */
+  int kernel_variant;           /* element-kernel form in use: 2 (column form) */
 } sfg_info3d;
 
 /* Reference: specfem::assembly::assembly<dim3> construction from the mesh. */
@@ -79,7 +78,7 @@ int sfg3d_run_timed_flushed(sfg_handle3d *h, int nsteps, size_t flush_bytes, flo
  * step's source-time values) copied in, the step's seismogram row
  * [ntypes][nrec][3] copied out; synchronous. */
 int sfg3d_step_io(sfg_handle3d *h, const float *stf_row, float *seis_row);
-/* Average duration of one launch of kernel `which` (0 element, 1 update). */
+/* Average duration of one launch of kernel `which` (0 layer kernel, 1 finish kernel). */
 int sfg3d_time_kernel(sfg_handle3d *h, int which, int reps, float *ms);
 int sfg3d_reset_fields(sfg_handle3d *h);
 int sfg3d_get_info(sfg_handle3d *h, sfg_info3d *info);

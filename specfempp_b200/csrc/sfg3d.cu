@@ -7,8 +7,7 @@
 // 4/3 mu, kappa = rho (vp^2 - 4/3 vs^2)), mass matrix rho w w w |J|
 // (include/medium/dim3/elastic/isotropic/mass_matrix.tpp:5-15), absorbing
 // faces, source arrays (compute_source_array/dim3/impl/*) and receiver
-// interpolants; the point-major contribution slots of the owner-computes
-// assembly.
+// interpolants.
 #include <cuda_runtime.h>
 #include <omp.h>
 
@@ -148,9 +147,13 @@ struct sfg_handle3d {
   int absorbing[6] = {0, 0, 0, 0, 0, 0};
   double zd[5], wd[5], hpd[5][5];
   // host set-up
-  std::vector<float> g9;  // [9][nloc]
-  std::vector<float> jac, c0, mu;
-  std::vector<int> slot, inv_start, bc_slot;
+  // |J| d xi_k / d x_j [9][nloc], or where every element is a box along the
+  // axes its three diagonal values an element
+  bool boxes = false;
+  std::vector<float> g9;
+  std::vector<float4> ediag;
+  std::vector<float> c0, mu;  // moduli / |J|
+  std::vector<int> bc_slot;
   std::vector<float> bc_c, minv;
   // sources / receivers
   std::vector<sfg_source3d> sources;
@@ -165,22 +168,26 @@ struct sfg_handle3d {
   int host_step = 0;
   // device
   std::unique_ptr<sfg3::DevMem> mem;
-  sfg3::dev::Elem3Args EA{};
+  sfg3::dev::Step3Args SA{};
   int *d_step = nullptr, *d_flag = nullptr;
-  float *d_u = nullptr, *d_v = nullptr, *d_a = nullptr, *d_minv = nullptr, *d_r = nullptr;
-  int *d_inv_start = nullptr, *d_ibool = nullptr, *d_rec_elem = nullptr, *d_types = nullptr;
+  // a step reads the fields of buffer par and writes the other's
+  float *d_u[2] = {nullptr, nullptr}, *d_v[2] = {nullptr, nullptr}, *d_a = nullptr;
+  int par = 0;
+  bool late = false;          // velocity or acceleration receivers
+  int *d_rec_elem = nullptr, *d_types = nullptr;
   float *d_rec_h = nullptr, *d_seis = nullptr, *d_stf = nullptr;
   float *flush = nullptr;
   size_t flush_bytes = 0;
-  int epb = 4;
+  int layers = 4;             // element layers a block of the layer kernel marches
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  cudaGraphExec_t graph_k = nullptr, graph_1 = nullptr, graph_e = nullptr;
-  int graph_steps = 20;
+  cudaGraphExec_t graph_k[2] = {}, graph_1[2] = {}, graph_e[2] = {};   // per buffer the first step reads
+  int graph_steps = 20;       // even: graph_k ends on the buffer it started from
   int sm_count = 148;
   ~sfg_handle3d() {
-    for (cudaGraphExec_t g : {graph_k, graph_1, graph_e})
-      if (g) cudaGraphExecDestroy(g);
+    for (int p = 0; p < 2; ++p)
+      for (cudaGraphExec_t g : {graph_k[p], graph_1[p], graph_e[p]})
+        if (g) cudaGraphExecDestroy(g);
     if (flush) cudaFree(flush);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -266,40 +273,74 @@ void locate(const sfg_handle3d *h, const double *X, int &elem, double xi[3]) {
 void setup_geometry(sfg_handle3d *h) {
   const size_t nloc = h->nloc;
   const int NX = 4 * h->nex + 1, NY = 4 * h->ney + 1;
-  h->g9.assign(9 * nloc, 0.0f);
-  h->jac.assign(nloc, 0.0f);
   h->c0.assign(nloc, 0.0f);
   h->mu.assign(nloc, 0.0f);
-  std::vector<int> ibool(nloc);
-  std::vector<double> mass(size_t(h->nglob), 0.0);
+  auto lattice = [&](int e, int q) {
+    const int ex = e % h->nex, ey = (e / h->nex) % h->ney, ez = e / (h->nex * h->ney);
+    return (size_t(4 * ez + q / (NG * NG)) * NY + 4 * ey + (q / NG) % NG) * NX + 4 * ex + q % NG;
+  };
+  // Boxes along the axes up to the rounding of their control nodes (1e-10 of
+  // the diagonal derivatives): such a mesh keeps three values an element.
+  bool boxes = true;
+#pragma omp parallel for schedule(static) reduction(&& : boxes)
+  for (int e = 0; e < h->nspec; ++e) {
+    if (!boxes) continue;
+    double cn[8][3];
+    corners(h, e, cn);
+    const sfg3::Geo C = sfg3::map_point(cn, 0, 0, 0);
+    for (int a = 0; a < 8; ++a) {
+      const sfg3::Geo G = sfg3::map_point(cn, sfg3::CS[a][0], sfg3::CS[a][1], sfg3::CS[a][2]);
+      for (int k = 0; k < 3; ++k)
+        for (int j = 0; j < 3; ++j) {
+          // inverse derivatives against the diagonal ones of their row and column
+          const double s = std::sqrt(std::fabs(C.inv[k][k] * C.inv[j][j]));
+          boxes = boxes && std::fabs(G.inv[k][j] - (k == j ? C.inv[k][k] : 0.0)) <= 1e-10 * s;
+        }
+    }
+  }
+  h->boxes = boxes;
+  if (boxes) h->ediag.resize(size_t(h->nspec));
+  else h->g9.assign(9 * nloc, 0.0f);
+  std::vector<double> wjac(nloc);   // |J|
   bool bad = false;
 #pragma omp parallel for schedule(static) reduction(|| : bad)
   for (int e = 0; e < h->nspec; ++e) {
     double cn[8][3];
     corners(h, e, cn);
-    const int ex = e % h->nex, ey = (e / h->nex) % h->ney, ez = e / (h->nex * h->ney);
+    const sfg3::Geo C = sfg3::map_point(cn, 0, 0, 0);
     for (int q = 0; q < NQ; ++q) {
       const int ix = q % NG, iy = (q / NG) % NG, iz = q / (NG * NG);
       const size_t p = size_t(e) * NQ + q;
-      ibool[p] = ((4 * ez + iz) * NY + 4 * ey + iy) * NX + 4 * ex + ix;
-      const sfg3::Geo G = sfg3::map_point(cn, h->zd[ix], h->zd[iy], h->zd[iz]);
+      const sfg3::Geo G = boxes ? C : sfg3::map_point(cn, h->zd[ix], h->zd[iy], h->zd[iz]);
       if (!(G.jac > 0)) bad = true;
-      for (int k = 0; k < 3; ++k)
-        for (int j = 0; j < 3; ++j) h->g9[size_t(k * 3 + j) * nloc + p] = float(G.inv[k][j]);
-      h->jac[p] = float(G.jac);
+      if (!boxes)
+        for (int k = 0; k < 3; ++k)
+          for (int j = 0; j < 3; ++j) h->g9[size_t(k * 3 + j) * nloc + p] = float(G.inv[k][j] * G.jac);
+      wjac[p] = G.jac;
       const double rho = h->rho[p], vp = h->vp[p], vs = h->vs[p];
       const double m = rho * vs * vs, kappa = rho * (vp * vp - 4.0 / 3.0 * vs * vs);
-      h->c0[p] = float(kappa + 4.0 / 3.0 * m);
-      h->mu[p] = float(m);
+      h->c0[p] = float((kappa + 4.0 / 3.0 * m) / G.jac);
+      h->mu[p] = float(m / G.jac);
     }
+    if (boxes)
+      h->ediag[size_t(e)] = make_float4(float(C.inv[0][0] * C.jac), float(C.inv[1][1] * C.jac),
+                                        float(C.inv[2][2] * C.jac), 0.f);
   }
+  // |J| grad xi_k at an element point
+  auto metric = [&](int e, int q, int k, double n[3]) {
+    for (int j = 0; j < 3; ++j) {
+      if (boxes) n[j] = j == k ? double((&h->ediag[size_t(e)].x)[k]) : 0.0;
+      else n[j] = double(h->g9[size_t(k * 3 + j) * nloc + size_t(e) * NQ + q]);
+    }
+  };
+  std::vector<double> mass(size_t(h->nglob), 0.0);
   if (bad) throw std::runtime_error("non-positive Jacobian in the mesh");
   // mass (serial: fixed summation order)
   for (int e = 0; e < h->nspec; ++e)
     for (int q = 0; q < NQ; ++q) {
       const size_t p = size_t(e) * NQ + q;
       const int ix = q % NG, iy = (q / NG) % NG, iz = q / (NG * NG);
-      mass[size_t(ibool[p])] += double(h->rho[p]) * h->wd[ix] * h->wd[iy] * h->wd[iz] * double(h->jac[p]);
+      mass[lattice(e, q)] += double(h->rho[p]) * h->wd[ix] * h->wd[iy] * h->wd[iz] * wjac[p];
     }
   // absorbing faces: per element point C = sum over the element's absorbing
   // faces of w_a w_b [(rvp - rvs) n n^T / |n| + rvs |n| I]; implicit mass term
@@ -329,7 +370,8 @@ void setup_geometry(sfg_handle3d *h) {
           const int q = (idx[2] * NG + idx[1]) * NG + idx[0];
           const size_t p = size_t(e) * NQ + q;
           double n[3];
-          for (int j = 0; j < 3; ++j) n[j] = sgn * double(h->g9[size_t(k * 3 + j) * h->nloc + p]) * double(h->jac[p]);
+          metric(e, q, k, n);
+          for (int j = 0; j < 3; ++j) n[j] *= sgn;
           const double nn = std::sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
           const double rho = h->rho[p], rvp = rho * double(h->vp[p]), rvs = rho * double(h->vs[p]);
           const double wab = h->wd[b] * h->wd[c];
@@ -344,7 +386,7 @@ void setup_geometry(sfg_handle3d *h) {
           const double vv = -h->opt.dt * 0.5, vn = vv * (n[0] + n[1] + n[2]);
           for (int j = 0; j < 3; ++j) {
             const double fj = (vn * n[j] / (nn * nn)) * (rvp - rvs) + vv * rvs;
-            mst[size_t(ibool[p]) * 3 + j] += -1.0 * fj * nn * wab;
+            mst[lattice(e, q) * 3 + j] += -1.0 * fj * nn * wab;
           }
         }
     }
@@ -353,16 +395,7 @@ void setup_geometry(sfg_handle3d *h) {
   h->minv.assign(size_t(h->nglob) * 3, 0.0f);
   for (size_t g = 0; g < size_t(h->nglob); ++g)
     for (int j = 0; j < 3; ++j) h->minv[g * 3 + j] = float(1.0 / (mass[g] + mst[g * 3 + j]));
-  // point-major slots: each point's contributions in increasing element order
-  h->inv_start.assign(size_t(h->nglob) + 1, 0);
-  for (size_t p = 0; p < nloc; ++p) h->inv_start[size_t(ibool[p]) + 1]++;
-  for (size_t g = 0; g < size_t(h->nglob); ++g) h->inv_start[g + 1] += h->inv_start[g];
-  std::vector<int> fill(h->inv_start.begin(), h->inv_start.end() - 1);
-  h->slot.resize(nloc);
-  for (size_t p = 0; p < nloc; ++p) h->slot[p] = fill[size_t(ibool[p])]++;
-  h->EA.nloc = nloc;
   h->mem.reset(new sfg3::DevMem());
-  h->d_ibool = h->mem->upload(ibool);
 }
 
 void setup_sources(sfg_handle3d *h) {
@@ -400,12 +433,14 @@ void setup_sources(sfg_handle3d *h) {
         for (int c = 0; c < 3; ++c) arr[c * NQ + q] = float(hl * S.comp[c]);
       }
     } else if (S.kind == SFG_SOURCE_MOMENT_TENSOR) {
-      double J[3][3] = {{0}};
+      double J[3][3] = {{0}}, cn[8][3];
+      corners(h, e, cn);
       for (int q = 0; q < NQ; ++q) {
         const int ix = q % NG, iy = (q / NG) % NG, iz = q / (NG * NG);
         const double hl = hh[0][ix] * hh[1][iy] * hh[2][iz];
+        const sfg3::Geo G = sfg3::map_point(cn, h->zd[ix], h->zd[iy], h->zd[iz]);
         for (int k = 0; k < 3; ++k)
-          for (int j = 0; j < 3; ++j) J[k][j] += hl * double(h->g9[size_t(k * 3 + j) * h->nloc + size_t(e) * NQ + q]);
+          for (int j = 0; j < 3; ++j) J[k][j] += hl * G.inv[k][j];
       }
       const double *cp = S.comp;
       const double M[3][3] = {{cp[0], cp[3], cp[4]}, {cp[3], cp[1], cp[5]}, {cp[4], cp[5], cp[2]}};
@@ -432,54 +467,65 @@ void setup_sources(sfg_handle3d *h) {
   }
 }
 
-// Element kernel launch: 1, 2 or 4 elements per block run the point form
-// (one thread per element point), 6 or 8 the column form (one thread per
-// column of five points).
-int col3_smem(int E) { return E * 9 * 25 * sfg3::dev::RP3 * int(sizeof(float)); }
+// Layers a block marches: the caller's elements_per_block (1, 2, 4, 6 or 8)
+// or the autotuner's pick; no choice changes a bit.
+bool valid_layers(int e) { return e == 1 || e == 2 || e == 4 || e == 6 || e == 8; }
 
-void launch_elem(sfg_handle3d *h, const sfg3::dev::Elem3Args &A, cudaStream_t s) {
-  const int E = h->epb;
-  const int grid = (h->nspec + E - 1) / E;
-  switch (E) {
-    case 1: sfg3::dev::k_stiffness3d<1><<<grid, NQ * 1, 0, s>>>(A); break;
-    case 2: sfg3::dev::k_stiffness3d<2><<<grid, NQ * 2, 0, s>>>(A); break;
-    case 6: sfg3::dev::k_stiffness3d_col<6><<<grid, 25 * 6, col3_smem(6), s>>>(A); break;
-    case 8: sfg3::dev::k_stiffness3d_col<8><<<grid, 25 * 8, col3_smem(8), s>>>(A); break;
-    default: sfg3::dev::k_stiffness3d<4><<<grid, NQ * 4, 0, s>>>(A); break;
-  }
+template <typename... P, typename... A>
+void launch_pdl(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(unsigned(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  SFG3_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
 }
 
-bool valid_epb3(int e) { return e == 1 || e == 2 || e == 4 || e == 6 || e == 8; }
+sfg3::dev::Step3Args step_args(const sfg_handle3d *h, bool predict, bool advance) {
+  sfg3::dev::Step3Args A = h->SA;
+  A.L = h->layers;
+  A.nchunk = (h->nez + h->layers - 1) / h->layers;
+  A.uo = h->d_u[h->par]; A.vo = h->d_v[h->par];
+  A.un = h->d_u[h->par ^ 1]; A.vn = h->d_v[h->par ^ 1];
+  A.a_store = !predict || h->late ? h->d_a : nullptr;
+  A.predict = predict ? 1 : 0;
+  A.advance = advance ? 1 : 0;
+  return A;
+}
 
+void launch_layers(const sfg_handle3d *h, const sfg3::dev::Step3Args &A, cudaStream_t s) {
+  const dim3 grid(unsigned(A.nbx * A.nby), unsigned(A.nchunk));
+  if (h->boxes) launch_pdl(sfg3::dev::k_layer3d<1>, grid, sfg3::dev::TILE_THREADS, sfg3::dev::L3_SMEM, s, A);
+  else launch_pdl(sfg3::dev::k_layer3d<0>, grid, sfg3::dev::TILE_THREADS, sfg3::dev::L3_SMEM, s, A);
+}
+
+void launch_finish(const sfg3::dev::Step3Args &A, cudaStream_t s) {
+  const int ntile = A.nbx * A.nby, planes = sfg3::dev::finish_planes(ntile, A.NZ), ngroup = (A.NZ + planes - 1) / planes;
+  launch_pdl(sfg3::dev::k_finish3d, dim3(unsigned(A.rec_blocks + ntile * (ngroup + A.nchunk - 1))), 256, 0, s, A);
+}
+
+// One step from buffer par into the other; par flips.
 void launch_step(sfg_handle3d *h, cudaStream_t s, bool predict) {
-  sfg3::dev::Elem3Args A = h->EA;
-  A.step = h->d_step;
-  launch_elem(h, A, s);
-  if (h->nrec) {
-    sfg3::dev::Rec3Args R{};
-    R.ibool = h->d_ibool; R.rec_elem = h->d_rec_elem; R.rec_h = h->d_rec_h; R.types = h->d_types;
-    R.ntypes = h->ntypes; R.nrec = h->nrec; R.nsig = h->opt.nstep;
-    R.u = h->d_u; R.v = h->d_v; R.minv = h->d_minv; R.r = h->d_r; R.inv_start = h->d_inv_start;
-    R.dt2 = float(h->opt.dt) / 2.0f;
-    R.step = h->d_step; R.seis = h->d_seis;
-    sfg3::dev::k_receivers3d<<<h->nrec, 128, 0, s>>>(R);
-  }
-  sfg3::dev::Update3Args U{};
-  U.u = h->d_u; U.v = h->d_v; U.a_store = predict ? nullptr : h->d_a;
-  U.minv = h->d_minv; U.inv_start = h->d_inv_start; U.r = h->d_r; U.npts = h->nglob;
-  const float dt = float(h->opt.dt);
-  U.dt = dt; U.dt2 = dt / 2.0f; U.dtsq2 = dt * dt / 2.0f;
-  U.predict = predict ? 1 : 0;
-  U.flag = h->d_flag; U.step = h->d_step; U.advance = 1;
-  const int ug = std::max(1, std::min((h->nglob + 255) / 256, h->sm_count * 8));
-  sfg3::dev::k_update3d<<<ug, 256, 0, s>>>(U);
+  const sfg3::dev::Step3Args A = step_args(h, predict, true);
+  launch_layers(h, A, s);
+  launch_finish(A, s);
+  if (h->late) launch_pdl(sfg3::dev::k_receivers3d, dim3(unsigned(h->nrec)), 128, 0, s, A);
+  h->par ^= 1;
 }
 
-cudaGraphExec_t capture(sfg_handle3d *h, int n, bool last_predicts) {
+cudaGraphExec_t capture(sfg_handle3d *h, int n, bool last_predicts, int par) {
   cudaGraph_t g = nullptr;
+  const int save = h->par;
+  h->par = par;
   SFG3_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   for (int i = 0; i < n; ++i) launch_step(h, h->stream, i + 1 < n || last_predicts);
   SFG3_CUDA(cudaStreamEndCapture(h->stream, &g));
+  h->par = save;
   cudaGraphExec_t ex = nullptr;
   SFG3_CUDA(cudaGraphInstantiate(&ex, g, 0));
   cudaGraphDestroy(g);
@@ -490,25 +536,48 @@ void resume(sfg_handle3d *h) {
   if (h->state_final) {
     const float dt = float(h->opt.dt);
     const size_t n = size_t(h->nglob) * 3;
-    sfg3::dev::k_predict3d<<<h->sm_count * 8, 256, 0, h->stream>>>(h->d_u, h->d_v, h->d_a, n, dt, dt / 2.0f,
+    sfg3::dev::k_predict3d<<<h->sm_count * 8, 256, 0, h->stream>>>(h->d_u[h->par], h->d_v[h->par], h->d_a, n, dt, dt / 2.0f,
                                                                       dt * dt / 2.0f);
     h->state_final = false;
+  }
+}
+
+// n steps that end on the next step's predictor.
+void run_fused(sfg_handle3d *h, int n) {
+  for (; n >= h->graph_steps; n -= h->graph_steps) SFG3_CUDA(cudaGraphLaunch(h->graph_k[h->par], h->stream));
+  for (; n > 0; --n) {
+    SFG3_CUDA(cudaGraphLaunch(h->graph_1[h->par], h->stream));
+    h->par ^= 1;
   }
 }
 
 void run_steps(sfg_handle3d *h, int n) {
   if (n <= 0) return;
   resume(h);
-  int fused = n - 1;
-  while (fused >= h->graph_steps) {
-    SFG3_CUDA(cudaGraphLaunch(h->graph_k, h->stream));
-    fused -= h->graph_steps;
-  }
-  for (; fused > 0; --fused) SFG3_CUDA(cudaGraphLaunch(h->graph_1, h->stream));
-  SFG3_CUDA(cudaGraphLaunch(h->graph_e, h->stream));
+  run_fused(h, n - 1);
+  SFG3_CUDA(cudaGraphLaunch(h->graph_e[h->par], h->stream));
+  h->par ^= 1;
   h->state_final = true;
   h->host_step += n;
   SFG3_CUDA(cudaGetLastError());
+}
+
+// Zero wavefields and seismograms, step 0, and wait.  (The buffer a step
+// writes needs no clearing.)
+int clear_fields(sfg_handle3d *h) {
+  const size_t n = (size_t(h->nglob) * 3 + 4) * sizeof(float);
+  h->par = 0;
+  SFG3_CUDA(cudaMemsetAsync(h->d_u[0], 0, n, h->stream));
+  SFG3_CUDA(cudaMemsetAsync(h->d_v[0], 0, n, h->stream));
+  SFG3_CUDA(cudaMemsetAsync(h->d_a, 0, n, h->stream));
+  SFG3_CUDA(cudaMemsetAsync(h->d_step, 0, 2 * sizeof(int), h->stream));
+  SFG3_CUDA(cudaMemsetAsync(h->d_flag, 0, sizeof(int), h->stream));
+  SFG3_CUDA(cudaMemsetAsync(h->d_seis, 0, size_t(h->opt.nstep) * h->ntypes * std::max(h->nrec, 1) * 3 * sizeof(float),
+                            h->stream));
+  SFG3_CUDA(cudaStreamSynchronize(h->stream));
+  h->state_final = true;
+  h->host_step = 0;
+  return SFG_OK;
 }
 
 }  // namespace
@@ -552,8 +621,8 @@ int sfg3d_create(const sfg_mesh3d_desc *mesh, const sfg_options *opt, sfg_handle
       g_create_error3 = "model values must give rho > 0, vs >= 0, lambda + 2 mu > 0";
       return SFG_ERR_ARG;
     }
-  if (valid_epb3(opt->elements_per_block)) h->epb = opt->elements_per_block;
-  if (opt->steps_per_graph > 0) h->graph_steps = opt->steps_per_graph;
+  if (valid_layers(opt->elements_per_block)) h->layers = opt->elements_per_block;
+  if (opt->steps_per_graph > 0) h->graph_steps = opt->steps_per_graph + opt->steps_per_graph % 2;
   *out = h.release();
   return SFG_OK;
 }
@@ -635,14 +704,25 @@ int sfg3d_initialize(sfg_handle3d *h) {
     SFG3_CUDA(cudaMemcpyToSymbol(sfg3::dev::c3_hp, hp, sizeof(hp)));
     SFG3_CUDA(cudaMemcpyToSymbol(sfg3::dev::c3_hpw, hpw, sizeof(hpw)));
     SFG3_CUDA(cudaMemcpyToSymbol(sfg3::dev::c3_w, w, sizeof(w)));
+    float rows[10][8] = {};
+    for (int i = 0; i < NG; ++i)
+      for (int l = 0; l < NG; ++l) {
+        rows[i][l] = hp[i * NG + l];
+        rows[5 + i][l] = hpw[l * NG + i];
+      }
+    SFG3_CUDA(cudaMemcpyToSymbol(sfg3::dev::t3_rows, rows, sizeof(rows)));
     sfg3::DevMem &m = *h->mem;
-    sfg3::dev::Elem3Args &A = h->EA;
-    A.ibool = h->d_ibool;
-    A.g9 = m.upload(h->g9);
-    A.jac = m.upload(h->jac);
+    sfg3::dev::Step3Args &A = h->SA;
+    A.nex = h->nex; A.ney = h->ney; A.nez = h->nez;
+    A.nbx = (h->nex + sfg3::dev::TX - 1) / sfg3::dev::TX;
+    A.nby = (h->ney + sfg3::dev::TY - 1) / sfg3::dev::TY;
+    A.NX = 4 * h->nex + 1; A.NY = 4 * h->ney + 1; A.NZ = 4 * h->nez + 1;
+    A.nloc = h->nloc;
+    if (h->boxes) A.ediag = m.upload(h->ediag);
+    else A.g9 = m.upload(h->g9);
     A.c0 = m.upload(h->c0);
     A.mu = m.upload(h->mu);
-    A.slot = m.upload(h->slot);
+    A.minv = m.upload(h->minv);
     A.bc_slot = m.upload(h->bc_slot);
     A.bc_c = h->bc_c.empty() ? nullptr : m.upload(h->bc_c);
     A.src_head = m.upload(h->src_head);
@@ -652,85 +732,81 @@ int sfg3d_initialize(sfg_handle3d *h) {
     A.stf = h->d_stf;
     A.nsrc = std::max(h->nsrc, 1);
     A.nstep = h->opt.nstep;
-    A.nspec = h->nspec;
-    A.nloc = h->nloc;
     const size_t n = size_t(h->nglob) * 3 + 4;
-    h->d_u = m.zeros<float>(n);
-    h->d_v = m.zeros<float>(n);
+    for (int p = 0; p < 2; ++p) {
+      h->d_u[p] = m.zeros<float>(n);
+      h->d_v[p] = m.zeros<float>(n);
+    }
     h->d_a = m.zeros<float>(n);
-    h->d_r = m.zeros<float>(h->nloc * 3 + 4);
-    h->d_minv = m.upload(h->minv);
-    h->d_inv_start = m.upload(h->inv_start);
-    A.u = h->d_u; A.v = h->d_v; A.r = h->d_r;
-    if (h->nsrc == 0) A.src_head = m.upload(std::vector<int>(size_t(h->nspec), -1));
     h->d_rec_elem = m.upload(h->rec_elem);
     h->d_rec_h = m.upload(h->rec_h);
     h->d_types = m.upload(h->types);
     h->d_seis = m.zeros<float>(size_t(h->opt.nstep) * h->ntypes * std::max(h->nrec, 1) * 3);
-    h->d_step = m.zeros<int>(1);
+    h->d_step = m.zeros<int>(2);
     h->d_flag = m.zeros<int>(1);
+    A.step = h->d_step; A.flag = h->d_flag;
+    A.rec_elem = h->d_rec_elem; A.rec_h = h->d_rec_h; A.types = h->d_types;
+    A.ntypes = h->ntypes; A.nrec = h->nrec; A.nsig = h->opt.nstep;
+    A.seis = h->d_seis;
+    bool early = false;
+    for (int t : h->types) (t == 0 ? early : h->late) = h->nrec > 0;
+    A.rec_blocks = early ? (h->nrec + 1) / 2 : 0;
+    const float dt = float(h->opt.dt);
+    A.dt = dt; A.dt2 = dt / 2.0f; A.dtsq2 = dt * dt / 2.0f;
     // host copies no longer needed
     std::vector<float>().swap(h->g9);
-    std::vector<float>().swap(h->jac);
     std::vector<float>().swap(h->c0);
     std::vector<float>().swap(h->mu);
-    std::vector<int>().swap(h->slot);
+    SFG3_CUDA(cudaFuncSetAttribute(sfg3::dev::k_layer3d<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   sfg3::dev::L3_SMEM));
+    SFG3_CUDA(cudaFuncSetAttribute(sfg3::dev::k_layer3d<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   sfg3::dev::L3_SMEM));
+    // the tiles' parts of shared points: sized for the shortest march tried
+    std::vector<int> cand;
+    if (valid_layers(h->opt.elements_per_block)) cand = {h->opt.elements_per_block};
+    else
+      for (int L : {1, 2, 4, 8, 16})
+        if (L == 1 || L < 2 * h->nez) cand.push_back(L);
+    const size_t ntile = size_t(A.nbx) * A.nby;
+    A.rim = m.zeros<float>(ntile * A.NZ * sfg3::dev::NEDGE * 3);
+    const size_t parts = ntile * size_t((h->nez + cand[0] - 1) / cand[0]) * sfg3::dev::NCOL * 3;
+    A.lower = m.zeros<float>(parts);
+    A.upper = m.zeros<float>(parts);
     SFG3_CUDA(cudaDeviceSynchronize());
-    SFG3_CUDA(cudaFuncSetAttribute(sfg3::dev::k_stiffness3d_col<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   col3_smem(8)));
-    SFG3_CUDA(cudaFuncSetAttribute(sfg3::dev::k_stiffness3d_col<6>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   col3_smem(6)));
-    if (!valid_epb3(h->opt.elements_per_block)) {
-      // launch-shape autotuner: elements per block and form of the element
-      // kernel, whole steps timed on this mesh (all shapes give the same bits)
+    h->layers = cand[0];
+    if (cand.size() > 1) {
+      // autotuner: layers a block marches, whole steps timed on this mesh (all
+      // give the same bits); few layers give more blocks, many give fewer
+      // points shared between blocks
       float best = 1e30f;
-      int pick = h->epb;
-      for (int e : {1, 2, 4, 6, 8}) {
-        h->epb = e;
+      int pick = cand[0];
+      for (int L : cand) {
+        h->layers = L;
         for (int i = 0; i < 2; ++i) launch_step(h, h->stream, true);
         SFG3_CUDA(cudaEventRecord(h->ev0, h->stream));
-        for (int i = 0; i < 3; ++i) launch_step(h, h->stream, true);
+        for (int i = 0; i < 4; ++i) launch_step(h, h->stream, true);
         SFG3_CUDA(cudaEventRecord(h->ev1, h->stream));
         SFG3_CUDA(cudaEventSynchronize(h->ev1));
         float t = 0;
         SFG3_CUDA(cudaEventElapsedTime(&t, h->ev0, h->ev1));
-        if (t < best) { best = t; pick = e; }
+        if (t < best) { best = t; pick = L; }
       }
-      h->epb = pick;
-      const size_t nb = n * sizeof(float);
-      SFG3_CUDA(cudaMemset(h->d_u, 0, nb));
-      SFG3_CUDA(cudaMemset(h->d_v, 0, nb));
-      SFG3_CUDA(cudaMemset(h->d_a, 0, nb));
-      SFG3_CUDA(cudaMemset(h->d_step, 0, sizeof(int)));
-      SFG3_CUDA(cudaMemset(h->d_flag, 0, sizeof(int)));
-      SFG3_CUDA(cudaMemset(h->d_seis, 0, size_t(h->opt.nstep) * h->ntypes * std::max(h->nrec, 1) * 3 * sizeof(float)));
-      SFG3_CUDA(cudaDeviceSynchronize());
+      h->layers = pick;
     }
-    h->graph_k = capture(h, h->graph_steps, true);
-    h->graph_1 = capture(h, 1, true);
-    h->graph_e = capture(h, 1, false);
+    for (int p = 0; p < 2; ++p) {
+      h->graph_k[p] = capture(h, h->graph_steps, true, p);
+      h->graph_1[p] = capture(h, 1, true, p);
+      h->graph_e[p] = capture(h, 1, false, p);
+    }
     h->initialized = true;
-    h->state_final = true;
-    h->host_step = 0;
-    return int(SFG_OK);
+    return clear_fields(h);
   });
 }
 
 int sfg3d_reset_fields(sfg_handle3d *h) {
   return guarded(h, [&]() {
     if (!h->initialized) { h->err = "sfg3d_initialize first"; return int(SFG_ERR_STATE); }
-    const size_t n = (size_t(h->nglob) * 3 + 4) * sizeof(float);
-    SFG3_CUDA(cudaMemsetAsync(h->d_u, 0, n, h->stream));
-    SFG3_CUDA(cudaMemsetAsync(h->d_v, 0, n, h->stream));
-    SFG3_CUDA(cudaMemsetAsync(h->d_a, 0, n, h->stream));
-    SFG3_CUDA(cudaMemsetAsync(h->d_step, 0, sizeof(int), h->stream));
-    SFG3_CUDA(cudaMemsetAsync(h->d_flag, 0, sizeof(int), h->stream));
-    SFG3_CUDA(cudaMemsetAsync(h->d_seis, 0, size_t(h->opt.nstep) * h->ntypes * std::max(h->nrec, 1) * 3 * sizeof(float),
-                              h->stream));
-    SFG3_CUDA(cudaStreamSynchronize(h->stream));
-    h->state_final = true;
-    h->host_step = 0;
-    return int(SFG_OK);
+    return clear_fields(h);
   });
 }
 
@@ -750,9 +826,7 @@ int sfg3d_run_timed(sfg_handle3d *h, int nsteps, float *ms) {
     if (nsteps <= 0 || h->host_step + nsteps > h->opt.nstep) { h->err = "beyond nstep"; return int(SFG_ERR_ARG); }
     resume(h);
     SFG3_CUDA(cudaEventRecord(h->ev0, h->stream));
-    int left = nsteps;
-    while (left >= h->graph_steps) { SFG3_CUDA(cudaGraphLaunch(h->graph_k, h->stream)); left -= h->graph_steps; }
-    for (; left > 0; --left) SFG3_CUDA(cudaGraphLaunch(h->graph_1, h->stream));
+    run_fused(h, nsteps);
     SFG3_CUDA(cudaEventRecord(h->ev1, h->stream));
     SFG3_CUDA(cudaEventSynchronize(h->ev1));
     SFG3_CUDA(cudaEventElapsedTime(ms, h->ev0, h->ev1));
@@ -795,7 +869,7 @@ int sfg3d_run_timed_flushed(sfg_handle3d *h, int nsteps, size_t flush_bytes, flo
                                                     flush_bytes / 16,
                                                     reinterpret_cast<float *>(fb + 2 * h->flush_bytes));
       SFG3_CUDA(cudaEventRecord(h->ev0, h->stream));
-      SFG3_CUDA(cudaGraphLaunch(h->graph_1, h->stream));
+      run_fused(h, 1);
       SFG3_CUDA(cudaEventRecord(h->ev1, h->stream));
       SFG3_CUDA(cudaEventSynchronize(h->ev1));
       float t = 0;
@@ -817,7 +891,7 @@ int sfg3d_step_io(sfg_handle3d *h, const float *stf_row, float *seis_row) {
       SFG3_CUDA(cudaMemcpyAsync(h->d_stf + size_t(step) * h->nsrc, stf_row, size_t(h->nsrc) * sizeof(float),
                                 cudaMemcpyHostToDevice, h->stream));
     resume(h);
-    SFG3_CUDA(cudaGraphLaunch(h->graph_1, h->stream));
+    run_fused(h, 1);
     h->host_step += 1;
     if (seis_row && h->nrec > 0)
       SFG3_CUDA(cudaMemcpyAsync(seis_row, h->d_seis + size_t(step) * h->ntypes * h->nrec * 3,
@@ -830,39 +904,19 @@ int sfg3d_step_io(sfg_handle3d *h, const float *stf_row, float *seis_row) {
 int sfg3d_time_kernel(sfg_handle3d *h, int which, int reps, float *ms) {
   return guarded(h, [&]() {
     if (!h->initialized || !ms || reps <= 0) return int(SFG_ERR_ARG);
-    // time on scratch copies of the mutable state: the fields are saved and restored
-    const size_t n = (size_t(h->nglob) * 3 + 4) * sizeof(float);
-    float *save = nullptr;
-    SFG3_CUDA(cudaMalloc(&save, 2 * n));
-    SFG3_CUDA(cudaMemcpyAsync(save, h->d_u, n, cudaMemcpyDeviceToDevice, h->stream));
-    SFG3_CUDA(cudaMemcpyAsync(reinterpret_cast<char *>(save) + n, h->d_v, n, cudaMemcpyDeviceToDevice, h->stream));
-    int step0 = 0;
-    SFG3_CUDA(cudaMemcpy(&step0, h->d_step, sizeof(int), cudaMemcpyDeviceToHost));
+    // the launches read the fields' buffers and write the other pair, which
+    // the next step overwrites: the state is as before
+    const sfg3::dev::Step3Args A = step_args(h, true, false);
     SFG3_CUDA(cudaEventRecord(h->ev0, h->stream));
     for (int i = 0; i < reps; ++i) {
-      if (which == 0) {
-        sfg3::dev::Elem3Args A = h->EA;
-        A.step = h->d_step;
-        launch_elem(h, A, h->stream);
-      } else {
-        sfg3::dev::Update3Args U{};
-        U.u = h->d_u; U.v = h->d_v; U.minv = h->d_minv; U.inv_start = h->d_inv_start; U.r = h->d_r;
-        U.npts = h->nglob; U.dt = float(h->opt.dt); U.dt2 = U.dt / 2; U.dtsq2 = U.dt * U.dt / 2;
-        U.predict = 1; U.flag = h->d_flag; U.step = h->d_step; U.advance = 0;
-        const int ug = std::max(1, std::min((h->nglob + 255) / 256, h->sm_count * 8));
-        sfg3::dev::k_update3d<<<ug, 256, 0, h->stream>>>(U);
-      }
+      if (which == 0) launch_layers(h, A, h->stream);
+      else launch_finish(A, h->stream);
     }
     SFG3_CUDA(cudaEventRecord(h->ev1, h->stream));
     SFG3_CUDA(cudaEventSynchronize(h->ev1));
     float t = 0;
     SFG3_CUDA(cudaEventElapsedTime(&t, h->ev0, h->ev1));
     *ms = t / reps;
-    SFG3_CUDA(cudaMemcpyAsync(h->d_u, save, n, cudaMemcpyDeviceToDevice, h->stream));
-    SFG3_CUDA(cudaMemcpyAsync(h->d_v, reinterpret_cast<char *>(save) + n, n, cudaMemcpyDeviceToDevice, h->stream));
-    SFG3_CUDA(cudaMemcpyAsync(h->d_step, &step0, sizeof(int), cudaMemcpyHostToDevice, h->stream));
-    SFG3_CUDA(cudaStreamSynchronize(h->stream));
-    cudaFree(save);
     return int(SFG_OK);
   });
 }
@@ -874,9 +928,9 @@ int sfg3d_get_info(sfg_handle3d *h, sfg_info3d *info) {
     info->nrec = h->nrec; info->ntypes = h->ntypes; info->nsig = h->opt.nstep; info->nsrc = h->nsrc;
     info->t0 = h->t0;
     info->device_bytes = h->mem ? h->mem->bytes : 0;
-    info->elements_per_block = h->epb;
-    info->kernels_per_step = 2 + (h->nrec > 0 ? 1 : 0);
-    info->kernel_variant = h->epb >= 6 ? 2 : 1;
+    info->elements_per_block = h->layers;
+    info->kernels_per_step = 2 + (h->late ? 1 : 0);
+    info->kernel_variant = 2;
     return int(SFG_OK);
   });
 }
@@ -899,7 +953,7 @@ int sfg3d_get_field(sfg_handle3d *h, int which, float *out, size_t count) {
     const size_t n = size_t(h->nglob) * 3;
     if (!out || count < n) { h->err = "output buffer too small"; return int(SFG_ERR_ARG); }
     if (!h->state_final) { h->err = "fields are mid-step after a timing call; run a step first"; return int(SFG_ERR_STATE); }
-    const float *src = which == 0 ? h->d_u : which == 1 ? h->d_v : h->d_a;
+    const float *src = which == 0 ? h->d_u[h->par] : which == 1 ? h->d_v[h->par] : h->d_a;
     SFG3_CUDA(cudaStreamSynchronize(h->stream));
     SFG3_CUDA(cudaMemcpy(out, src, n * sizeof(float), cudaMemcpyDeviceToHost));
     return int(SFG_OK);
