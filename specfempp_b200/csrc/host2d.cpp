@@ -538,6 +538,10 @@ void assemble_model2d(const Mesh2D &m, Assembly2D &a) {
   auto cos_of = [&](int e) { return &m.mat_cosserat[size_t(m.kmato[e]) * 8]; };
   if (a.el.aniso && (a.el.ncomp != 2 || !m.prho.empty()))
     throw std::runtime_error("anisotropic media: P-SV with material constants only (no SH, no point models)");
+  // a bad poroelastic material throws here, not inside a parallel loop
+  if (a.el.poro)
+    for (int ce = 0; ce < a.el.nspec; ++ce)
+      if (ce == 0 || m.kmato[a.el.elem_mesh[ce]] != m.kmato[a.el.elem_mesh[ce - 1]]) poro_words(poro_of(a.el.elem_mesh[ce]));
   for (int med = 0; med < 2; ++med) {
     MediumData &D = med == 1 ? a.el : a.ac;
     const size_t n = size_t(D.nspec) * NPTS;
@@ -548,6 +552,7 @@ void assemble_model2d(const Mesh2D &m, Assembly2D &a) {
     for (auto *v : {&D.prop6, &D.prop7, &D.prop8}) v->assign(med == 1 && D.poro ? n : 0, 0.0f);
     if (med == 1 && D.poro)
       for (auto *v : {&D.prop2, &D.prop3, &D.prop4, &D.prop5}) v->assign(n, 0.0f);
+#pragma omp parallel for schedule(static)
     for (int ce = 0; ce < D.nspec; ++ce) {
       const int e = D.elem_mesh[ce];
       for (int q = 0; q < NPTS; ++q) {
@@ -675,56 +680,57 @@ void assemble_model2d(const Mesh2D &m, Assembly2D &a) {
   // (compute_mass_matrix.tpp:95-121, stacey.tpp:817-853), then 1/M.
   for (int med = 0; med < 2; ++med) {
     MediumData &D = med == 1 ? a.el : a.ac;
-    std::vector<double> M(size_t(D.nglob) * D.ncomp, 0.0);
-    for (int ce = 0; ce < D.nspec; ++ce) {
-      const int e = D.elem_mesh[ce];
-      for (int iz = 0; iz < NGLL; ++iz)
-        for (int ix = 0; ix < NGLL; ++ix) {
-          const int q = iz * NGLL + ix;
-          const size_t pc = size_t(ce) * NPTS + q, pm = size_t(e) * NPTS + q;
-          const double fac = w[ix] * w[iz] * a.jac_d[pm];
-          double rho, vp, vs;
-          model(e, pm, rho, vp, vs);
-          double mc[4] = {0, 0, 0, 0};
-          if (med == 1) mc[0] = mc[1] = rho * fac;
-          else mc[0] = (1.0 / double(D.prop1[pc])) * fac;
-          if (med == 1 && D.poro) {
-            // solid rho_bar - phi rho_f / tort, fluid (rho_f tort rho_bar -
-            // phi rho_f^2) / (phi rho_bar) (poroelastic/isotropic/mass_matrix.tpp)
-            const double *v = poro_of(e);
-            const double phi = v[2], rhof = v[1], tort = v[3], rb = (1.0 - phi) * v[0] + phi * rhof;
-            mc[0] = mc[1] = (rb - phi * rhof / tort) * fac;
-            mc[2] = mc[3] = ((rhof * tort * rb - phi * rhof * rhof) / (phi * rb)) * fac;
-          }
-          // Cosserat: rho, rho, j (isotropic_cosserat/mass_matrix.tpp)
-          if (med == 1 && D.cosserat) mc[2] = m.mat_cosserat[size_t(m.kmato[e]) * 8 + 4] * fac;
-          if (D.bc_slot[ce] >= 0) {
-            const size_t k = size_t(D.bc_slot[ce]) * NPTS + q;
-            if (D.bc_w[k] != 0.0f) {
-              const double vv = -dt * 0.5;  // velocity stand-in of the implicit term
-              const double nx = D.bc_nx[k], nz = D.bc_nz[k], j1 = D.bc_j1[k], wq = D.bc_w[k];
-              if (med == 0) {
-                mc[0] += -1.0 * wq * j1 * double(D.bc_imp0[k]) * vv;
-              } else if (D.ncomp == 1) {
-                mc[0] += -1.0 * wq * j1 * double(D.bc_imp1[k]) * vv;
-              } else {
-                const double vn = vv * nx + vv * nz;
-                const double dn[2] = {nx, nz};
-                for (int c = 0; c < 2; ++c) {
-                  const double f = ((vn * dn[c] / (j1 * j1)) * (double(D.bc_imp0[k]) - double(D.bc_imp1[k]))) +
-                                   vv * double(D.bc_imp1[k]);
-                  mc[c] += -1.0 * f * j1 * wq;
-                }
-                if (D.cosserat) mc[2] += -1.0 * double(D.bc_imp2[k]) * vv * j1 * wq;
-              }
-            }
-          }
-          const int g = D.ibool[pc];
-          for (int c = 0; c < D.ncomp; ++c) M[size_t(g) * D.ncomp + c] += mc[c];
+    D.minv.resize(size_t(D.nglob) * D.ncomp);
+    // mass of one element point
+    auto point_mass = [&](size_t pc, double mc[4]) {
+      const int ce = int(pc / NPTS), q = int(pc % NPTS), e = D.elem_mesh[ce];
+      const size_t pm = size_t(e) * NPTS + q;
+      const double fac = w[q % NGLL] * w[q / NGLL] * a.jac_d[pm];
+      double rho, vp, vs;
+      model(e, pm, rho, vp, vs);
+      if (med == 1) mc[0] = mc[1] = rho * fac;
+      else mc[0] = (1.0 / double(D.prop1[pc])) * fac;
+      if (med == 1 && D.poro) {
+        // solid rho_bar - phi rho_f / tort, fluid (rho_f tort rho_bar -
+        // phi rho_f^2) / (phi rho_bar) (poroelastic/isotropic/mass_matrix.tpp)
+        const double *v = poro_of(e);
+        const double phi = v[2], rhof = v[1], tort = v[3], rb = (1.0 - phi) * v[0] + phi * rhof;
+        mc[0] = mc[1] = (rb - phi * rhof / tort) * fac;
+        mc[2] = mc[3] = ((rhof * tort * rb - phi * rhof * rhof) / (phi * rb)) * fac;
+      }
+      // Cosserat: rho, rho, j (isotropic_cosserat/mass_matrix.tpp)
+      if (med == 1 && D.cosserat) mc[2] = m.mat_cosserat[size_t(m.kmato[e]) * 8 + 4] * fac;
+      if (D.bc_slot[ce] < 0) return;
+      const size_t k = size_t(D.bc_slot[ce]) * NPTS + q;
+      if (D.bc_w[k] == 0.0f) return;
+      const double vv = -dt * 0.5;  // velocity stand-in of the implicit term
+      const double nx = D.bc_nx[k], nz = D.bc_nz[k], j1 = D.bc_j1[k], wq = D.bc_w[k];
+      if (med == 0) {
+        mc[0] += -1.0 * wq * j1 * double(D.bc_imp0[k]) * vv;
+      } else if (D.ncomp == 1) {
+        mc[0] += -1.0 * wq * j1 * double(D.bc_imp1[k]) * vv;
+      } else {
+        const double vn = vv * nx + vv * nz;
+        const double dn[2] = {nx, nz};
+        for (int c = 0; c < 2; ++c) {
+          const double f = ((vn * dn[c] / (j1 * j1)) * (double(D.bc_imp0[k]) - double(D.bc_imp1[k]))) +
+                           vv * double(D.bc_imp1[k]);
+          mc[c] += -1.0 * f * j1 * wq;
         }
+        if (D.cosserat) mc[2] += -1.0 * double(D.bc_imp2[k]) * vv * j1 * wq;
+      }
+    };
+    // each point sums its contributions in increasing compute order
+#pragma omp parallel for schedule(static)
+    for (int g = 0; g < D.nglob; ++g) {
+      double M[4] = {0, 0, 0, 0};
+      for (int k = D.inv_start[g]; k < D.inv_start[g + 1]; ++k) {
+        double mc[4] = {0, 0, 0, 0};
+        point_mass(size_t(D.inv_idx[k]), mc);
+        for (int c = 0; c < D.ncomp; ++c) M[c] += mc[c];
+      }
+      for (int c = 0; c < D.ncomp; ++c) D.minv[size_t(g) * D.ncomp + c] = float(1.0 / M[c]);
     }
-    D.minv.resize(M.size());
-    for (size_t i = 0; i < M.size(); ++i) D.minv[i] = float(1.0 / M[i]);
   }
   classify_rows(a.el);
   classify_rows(a.ac);
@@ -760,9 +766,12 @@ void set_model2d(Mesh2D &m, Assembly2D &a, const float *rho, const float *kappa,
   m.prho.resize(n);
   m.pvp.resize(n);
   m.pvs.resize(n);
+  bool bad = false;
+#pragma omp parallel for schedule(static) reduction(|| : bad)
+  for (size_t p = 0; p < n; ++p) bad = bad || !(rho[p] > 0) || !(mu[p] >= 0) || !(kappa[p] + 4.0 / 3.0 * mu[p] > 0);
+  if (bad) throw std::runtime_error("model values must give rho > 0, mu >= 0, lambda + 2 mu > 0");
+#pragma omp parallel for schedule(static)
   for (size_t p = 0; p < n; ++p) {
-    if (!(rho[p] > 0) || !(mu[p] >= 0) || !(kappa[p] + 4.0 / 3.0 * mu[p] > 0))
-      throw std::runtime_error("model values must give rho > 0, mu >= 0, lambda + 2 mu > 0");
     m.prho[p] = rho[p];
     m.pvs[p] = float(std::sqrt(double(mu[p]) / rho[p]));
     m.pvp[p] = float(std::sqrt((double(kappa[p]) + 4.0 / 3.0 * double(mu[p])) / rho[p]));
@@ -841,19 +850,23 @@ void assemble2d(const Mesh2D &m, double dt, Assembly2D &a) {
   std::vector<JacD> J(nloc);
   a.gx.resize(nloc);
   a.gz.resize(nloc);
+  bool folded = false;
+#pragma omp parallel for schedule(static) reduction(|| : folded)
   for (int e = 0; e < nspec; ++e)
     for (int iz = 0; iz < NGLL; ++iz)
       for (int ix = 0; ix < NGLL; ++ix) {
         const size_t p = size_t(e) * NPTS + iz * NGLL + ix;
         J[p] = jacobian(m, e, z[ix], z[iz]);
-        if (!(J[p].jac > 0)) throw std::runtime_error("non-positive Jacobian: check element orientation");
+        folded = folded || !(J[p].jac > 0);
         a.gx[p] = J[p].x;
         a.gz[p] = J[p].z;
       }
+  if (folded) throw std::runtime_error("non-positive Jacobian: check element orientation");
   // An element that is a rectangle along the axes up to the rounding of its
   // control nodes (1e-10 of its derivatives, far below the FP32 words that
   // the kernels read) gets exactly that geometry: zero cross derivatives and
   // one value of the others.
+#pragma omp parallel for schedule(static)
   for (int e = 0; e < nspec; ++e) {
     JacD *E = &J[size_t(e) * NPTS];
     const JacD C = E[NPTS / 2];

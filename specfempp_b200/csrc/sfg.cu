@@ -992,7 +992,7 @@ std::vector<unsigned char> tile_records(const sfg::MediumData &M, const std::vec
 }
 
 void refresh_tile_records(sfg_handle *h) {
-  if (!h->tile_ok) return;
+  if (!h->tile_ok || h->variant != 5) return;     // read by the fused tile kernels only
   for (int med = 0; med < 2; ++med) {
     DevMedium &D = med == 1 ? h->el : h->ac;
     const sfg::MediumData &M = med == 1 ? h->asmb.el : h->asmb.ac;
@@ -3074,6 +3074,7 @@ int sfg_adjoint_gradient(sfg_handle *h, const float *seis_grad, float *grad_rho,
       const float *tot = h->adj.h_stage;
       SFG_CUDA(cudaMemcpy(h->adj.h_stage, A.sum, A.nsum() * sizeof(float), cudaMemcpyDeviceToHost));
       const float *grho = tot + 2 * A.nloc;
+#pragma omp parallel for schedule(static)
       for (int ce = 0; ce < D.nspec; ++ce) {
         const int e = M.elem_mesh[ce];
         for (int q = 0; q < sfg::NPTS; ++q) {
