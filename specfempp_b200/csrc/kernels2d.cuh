@@ -494,8 +494,9 @@ __device__ __forceinline__ void acoustic_block(const StiffArgs &S, const MedArgs
 // colour, the following ac.nblocks blocks acoustic ones.
 // occupancy held at the warp limit of an SM (64 warps): the kernel is bound
 // by memory latency, so registers may not grow past what that allows
+struct RecPoint;
 template <bool EARLY>
-__device__ void receiver_warp(const RecArgs &A, int i, int lane, float *sf);
+__device__ void receiver_warp(const RecArgs &A, int i, int lane, float *sf, const RecPoint *P);
 
 // The first rec_blocks blocks of an element launch: one receiver a warp.
 __device__ __noinline__ void receiver_blocks(const RecArgs *ac, const RecArgs *el, int nac, int nel, float *smem) {
@@ -504,8 +505,8 @@ __device__ __noinline__ void receiver_blocks(const RecArgs *ac, const RecArgs *e
   pdl_release();
   const int i = blockIdx.x * nw + w;
   if (w >= nw || i >= nac + nel) return;
-  if (i < nac) receiver_warp<true>(*ac, i, lane, smem + w * 3 * NP);
-  else receiver_warp<true>(*el, i - nac, lane, smem + w * 3 * NP);
+  if (i < nac) receiver_warp<true>(*ac, i, lane, smem + w * 3 * NP, nullptr);
+  else receiver_warp<true>(*el, i - nac, lane, smem + w * 3 * NP, nullptr);
 }
 
 __device__ void save_stacey_velocity(const StiffArgs &S);
@@ -1132,9 +1133,24 @@ __device__ __forceinline__ float rec_accel(const RecArgs &A, int g, int c) {
 // accumulator (plus the coupling term on interface points).
 // EARLY: types that read only the displacement, taken inside the element
 // launch (whose other blocks are writing the contributions).  sf: 3 x 25
-// floats of the warp.
+// floats of the warp.  P: what a late receiver of the owner-computes step
+// loaded of its point before the wait (null: load and sum on demand).
+struct RecPoint {
+  int k0, k1;
+  float mi[2], v[2];
+};
+
+// Acceleration of component c (< 2) at point g.
+__device__ __forceinline__ float rec_accel(const RecArgs &A, const RecPoint *P, int g, int c) {
+  if (!P) return rec_accel(A, g, c);
+  float acc = 0.f;
+  for (int j = P->k0; j < P->k1; ++j) acc = acc + ld_dep(A.cpl.r + size_t(j) * A.ncomp + c);
+  if (g < A.cpl.niface) acc += coupling_term(A.cpl, g, c);
+  return __fmul_rn(acc, c ? P->mi[1] : P->mi[0]);
+}
+
 template <bool EARLY>
-__device__ void receiver_warp(const RecArgs &A, int i, int lane, float *sfp) {
+__device__ void receiver_warp(const RecArgs &A, int i, int lane, float *sfp, const RecPoint *P) {
   float (*sf)[NP] = reinterpret_cast<float (*)[NP]>(sfp);
   int isig = A.isig_fixed;
   if (isig < 0) {
@@ -1208,13 +1224,16 @@ __device__ void receiver_warp(const RecArgs &A, int i, int lane, float *sfp) {
       } else if (ty == 4) {                    // Cosserat rotation
         o[0] = warp_sum(nc == 3 ? h * ld_dep(A.u + size_t(g) * 3 + 2) : 0.f);
       } else {
-        for (int c = 0; c < (nc < 2 ? nc : 2); ++c) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          if (c >= nc) break;
           const size_t k = size_t(g) * A.ncomp + c;
+          const float vel = P ? P->v[c] : 0.f;
           float val = 0.f;
           switch (A.types[t]) {
             case 0: val = ld_dep(A.u + k); break;
-            case 1: if (!EARLY) val = A.final_fields ? A.v[k] : newmark_correct(ld_dep(A.v + k), rec_accel(A, g, c), A.dt2); break;
-            default: if (!EARLY) val = A.final_fields ? A.a[k] : rec_accel(A, g, c); break;
+            case 1: if (!EARLY) val = A.final_fields ? A.v[k] : newmark_correct(P ? vel : ld_dep(A.v + k), rec_accel(A, P, g, c), A.dt2); break;
+            default: if (!EARLY) val = A.final_fields ? A.a[k] : rec_accel(A, P, g, c); break;
           }
           o[c] = warp_sum(h * val);
         }
@@ -1228,10 +1247,10 @@ __device__ void receiver_warp(const RecArgs &A, int i, int lane, float *sfp) {
     return;
   }
   // acoustic: displacement-like outputs are rho^-1 grad(field); pressure = -chi_dd
-  const float a = EARLY ? 0.f : (A.final_fields ? A.a[g] : rec_accel(A, g, 0));
+  const float a = EARLY ? 0.f : (A.final_fields ? A.a[g] : rec_accel(A, P, g, 0));
   if (on) {
     sf[0][q] = ld_dep(A.u + g);
-    sf[1][q] = EARLY ? 0.f : (A.final_fields ? A.v[g] : newmark_correct(ld_dep(A.v + g), a, A.dt2));
+    sf[1][q] = EARLY ? 0.f : (A.final_fields ? A.v[g] : newmark_correct(P ? P->v[0] : ld_dep(A.v + g), a, A.dt2));
     sf[2][q] = a;
   }
   __syncwarp();
@@ -1267,9 +1286,27 @@ __device__ void receiver_warp(const RecArgs &A, int i, int lane, float *sfp) {
 
 __global__ void __launch_bounds__(32) k_receivers(const __grid_constant__ RecArgs A) {
   __shared__ float sf[3 * NP];
+  // The chain receiver -> element -> point -> fields before the wait: only
+  // the contributions are left after it.
+  if (A.cpl.inv_start && !A.final_fields) {
+    const int q = threadIdx.x < NP ? threadIdx.x : 0;
+    const int g = A.ibool[size_t(A.rec_elem[A.rec_list[blockIdx.x]]) * NP + q];
+    RecPoint P;
+    P.k0 = A.cpl.inv_start[g];
+    P.k1 = A.cpl.inv_start[g + 1];
+    const size_t o = size_t(g) * A.ncomp;
+    P.mi[0] = A.minv[o];
+    P.v[0] = ld_l2(A.v + o);
+    P.mi[1] = A.ncomp > 1 ? A.minv[o + 1] : 0.f;
+    P.v[1] = A.ncomp > 1 ? ld_l2(A.v + o + 1) : 0.f;
+    pdl_wait();
+    pdl_release();
+    receiver_warp<false>(A, blockIdx.x, threadIdx.x, sf, &P);
+    return;
+  }
   pdl_wait();
   pdl_release();
-  receiver_warp<false>(A, blockIdx.x, threadIdx.x, sf);
+  receiver_warp<false>(A, blockIdx.x, threadIdx.x, sf, nullptr);
 }
 
 }  // namespace dev
