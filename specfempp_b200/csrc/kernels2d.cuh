@@ -927,6 +927,12 @@ __device__ __forceinline__ bool update_point_post(const UpdateArgs &A, int g, Po
       const float2 t = ld_dep2(A.r + size_t(k) * 2);
       acc[0] = acc[0] + t.x;
       acc[NC - 1] = acc[NC - 1] + t.y;
+    } else if (NC == 4) {
+      const float4 t = ld_dep4(A.r + size_t(k) * 4);
+      acc[0] = acc[0] + t.x;
+      acc[1 % NC] = acc[1 % NC] + t.y;
+      acc[2 % NC] = acc[2 % NC] + t.z;
+      acc[3 % NC] = acc[3 % NC] + t.w;
     } else {
 #pragma unroll
       for (int c = 0; c < NC; ++c) acc[c] = acc[c] + ld_dep(A.r + size_t(k) * NC + c);
@@ -936,7 +942,13 @@ __device__ __forceinline__ bool update_point_post(const UpdateArgs &A, int g, Po
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[c] += coupling_term(A, g, c);
   }
-  if (NC > 2) {
+  if (NC == 4) {
+    const float4 u4 = ld_dep4(A.u + size_t(g) * 4), v4 = ld_dep4(A.v + size_t(g) * 4);
+    const float4 m4 = __ldg(reinterpret_cast<const float4 *>(A.minv) + g);
+    P.u[0] = u4.x; P.u[1 % NC] = u4.y; P.u[2 % NC] = u4.z; P.u[3 % NC] = u4.w;
+    P.v[0] = v4.x; P.v[1 % NC] = v4.y; P.v[2 % NC] = v4.z; P.v[3 % NC] = v4.w;
+    P.mi[0] = m4.x; P.mi[1 % NC] = m4.y; P.mi[2 % NC] = m4.z; P.mi[3 % NC] = m4.w;
+  } else if (NC > 2) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const size_t i = size_t(g) * NC + c;
@@ -965,6 +977,11 @@ __device__ __forceinline__ bool update_point_post(const UpdateArgs &A, int g, Po
     if (A.predict) reinterpret_cast<float2 *>(A.u)[g] = make_float2(P.u[0], P.u[NC - 1]);
     reinterpret_cast<float2 *>(A.v)[g] = make_float2(P.v[0], P.v[NC - 1]);
     if (A.a_store) reinterpret_cast<float2 *>(A.a_store)[g] = make_float2(a[0], a[NC - 1]);
+  } else if (NC == 4) {
+    if (A.predict)
+      reinterpret_cast<float4 *>(A.u)[g] = make_float4(P.u[0], P.u[1 % NC], P.u[2 % NC], P.u[3 % NC]);
+    reinterpret_cast<float4 *>(A.v)[g] = make_float4(P.v[0], P.v[1 % NC], P.v[2 % NC], P.v[3 % NC]);
+    if (A.a_store) reinterpret_cast<float4 *>(A.a_store)[g] = make_float4(a[0], a[1 % NC], a[2 % NC], a[3 % NC]);
   } else {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
