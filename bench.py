@@ -59,6 +59,21 @@ STEP_B_GLOB = 56
 STEP_B_LOCAL = 32
 
 
+def row_words(w):
+    """Geometry and material words an element point that the row-form element
+    kernel (variant 6) reads: none of either where they are one value an
+    element (axis-aligned rectangles, material constants), which it takes from
+    a 32-byte record an element."""
+    import numpy as np
+    m = w.mesh
+    c = np.asarray(m.coorg)[np.asarray(m.knods)[:, :4]]          # corners counter-clockwise from the lower left
+    h = np.abs(c[:, 2] - c[:, 0])
+    tilt = np.abs(np.stack([c[:, 1, 1] - c[:, 0, 1], c[:, 2, 1] - c[:, 3, 1], c[:, 3, 0] - c[:, 0, 0],
+                            c[:, 2, 0] - c[:, 1, 0]], 1))
+    straight = bool((tilt <= 1e-10 * h.min(axis=1)[:, None]).all()) and int(m.ngnod) == 4
+    return (0 if straight else 5), (0 if w.point_vp is None else 2)
+
+
 def peaks():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -332,7 +347,7 @@ def bench_3d(args, world, barrier, max_over_ranks):
     Stacey on the other faces, moment tensor (1 Hz), 1000 surface receivers,
     dt = 2 ms.  A bounded run of the 5000-step configuration: 10 warm-up steps,
     then K steps back to back (CUDA events, graph replay) and K steps each after
-    a 256 MiB L2 flush; model state (about 12.6 GB) far larger than L2."""
+    a 256 MiB L2 flush; model state (about 7 GB) far larger than L2."""
     from specfempp_b200 import meshgen, sfg3d
     nx, ny, nz = (int(v) for v in args.mesh3d.split("x"))
     steps = args.steps3d
@@ -352,7 +367,9 @@ def bench_3d(args, world, barrier, max_over_ranks):
     upd = sim.time_kernel(1, 10)
     finite = sim.check_finite()
     r = 125.0 * inf.nspec / inf.nglob
-    alg = 84.0 + 52.0 * r                       # algorithmic bytes per point-step
+    # algorithmic bytes per point-step: u and v read and written, M^-1 read (60),
+    # two moduli an element point (the mesh is boxes: three metric words an element)
+    alg = 60.0 + 8.0 * r
     peak, _ = peaks()
     out = {"workload": f"elastic3d_{nx}x{ny}x{nz}", "nglob": inf.nglob, "nspec": inf.nspec,
            "elements_per_block": inf.elements_per_block, "kernel_variant": inf.kernel_variant,
@@ -573,8 +590,16 @@ def main():
     stiff_ms_b2b = sim.time_kernel(0, 50)
     upd_ms = sim.time_kernel(1, 50)
     ac_ms = sim.time_kernel(2, 50)
-    if inf.kernel_variant >= 3:
-        # owner-computes (variants 3, 4, 6; for the fused tile kernel, 5, the
+    if inf.kernel_variant == 6:
+        # row form: indices of the point and of its contribution (8), what the
+        # mesh leaves per point, the contribution written (8 B elastic, 4 B
+        # acoustic), a record an element, the gathered field
+        geo, mat = row_words(w)
+        per = 8 + 4 * (geo + mat)
+        stiff_bytes = ((per + 8) * inf.nspec_elastic * 25 + 8 * inf.nglob_elastic +
+                       (per + 4) * inf.nspec_acoustic * 25 + 4 * inf.nglob_acoustic + 32 * inf.nspec)
+    elif inf.kernel_variant >= 3:
+        # owner-computes (variants 3, 4; for the fused tile kernel, 5, the
         # element part): the element kernel reads geometry and the gathered field
         # and writes each element point's contribution once (8 B elastic, 4 B acoustic)
         stiff_bytes = ((STIFF_B_PER_LOCAL + 8) * inf.nspec_elastic * 25 + 8 * inf.nglob_elastic +
@@ -589,7 +614,9 @@ def main():
     if tr and tr.get("workload") == args.workload:
         # the DRAM traffic of the element kernel in use, from its ncu capture
         traffic = tr.get("stiffness_bytes_per_launch_by_variant", {}).get(str(inf.kernel_variant))
-    step_bytes = STEP_B_GLOB * nglob + STEP_B_LOCAL * inf.nspec * 25
+    # a step of the row form reads no geometry or material word that is one value an element
+    step_local = STEP_B_LOCAL if inf.kernel_variant != 6 else 4 + 4 * sum(row_words(w))
+    step_bytes = STEP_B_GLOB * nglob + step_local * inf.nspec * 25
     kname = ("element kernel, one owner-computes launch of one step" if inf.kernel_variant >= 3 else
              f"element kernel, all {inf.ncolors_elastic} colour launches of one step")
     roofline = {"bound": "hbm", "kernel": f"{kname} (variant {inf.kernel_variant}, "
