@@ -764,6 +764,7 @@ struct UpdateArgs {
   float *__restrict__ u, *__restrict__ v, *__restrict__ accum;
   const float *__restrict__ minv;
   float *__restrict__ a_store;   // copy of the new acceleration (optional when predicting)
+  int a_n;                       // gather form: points whose acceleration is stored (the first a_n)
   int n;                         // nglob * ncomp
   int ncomp;
   // coupling: the first niface points take cp_n . other[cp_other] (acoustic
@@ -976,19 +977,19 @@ __device__ __forceinline__ bool update_point_post(const UpdateArgs &A, int g, Po
   if (NC == 2) {
     if (A.predict) reinterpret_cast<float2 *>(A.u)[g] = make_float2(P.u[0], P.u[NC - 1]);
     reinterpret_cast<float2 *>(A.v)[g] = make_float2(P.v[0], P.v[NC - 1]);
-    if (A.a_store) reinterpret_cast<float2 *>(A.a_store)[g] = make_float2(a[0], a[NC - 1]);
+    if (g < A.a_n) reinterpret_cast<float2 *>(A.a_store)[g] = make_float2(a[0], a[NC - 1]);
   } else if (NC == 4) {
     if (A.predict)
       reinterpret_cast<float4 *>(A.u)[g] = make_float4(P.u[0], P.u[1 % NC], P.u[2 % NC], P.u[3 % NC]);
     reinterpret_cast<float4 *>(A.v)[g] = make_float4(P.v[0], P.v[1 % NC], P.v[2 % NC], P.v[3 % NC]);
-    if (A.a_store) reinterpret_cast<float4 *>(A.a_store)[g] = make_float4(a[0], a[1 % NC], a[2 % NC], a[3 % NC]);
+    if (g < A.a_n) reinterpret_cast<float4 *>(A.a_store)[g] = make_float4(a[0], a[1 % NC], a[2 % NC], a[3 % NC]);
   } else {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const size_t i = size_t(g) * NC + c;
       if (A.predict) A.u[i] = P.u[c];
       A.v[i] = P.v[c];
-      if (A.a_store) A.a_store[i] = a[c];
+      if (g < A.a_n) A.a_store[i] = a[c];
     }
   }
   return bad;
