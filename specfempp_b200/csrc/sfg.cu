@@ -740,12 +740,11 @@ sfg::dev::UpdateArgs update_args(sfg_handle *h, const DevMedium &D, const DevMed
   return U;
 }
 
-// Update of a chained step: twice the resident blocks for one or two
-// components (the blocks then end one after another and leave room for the
-// next kernel's first ones: fluid-solid 400x200 step 30.7 -> 28.8 us), the
-// resident ones for three and four (fewer registers to spare: 18.8 against
-// 19.3 us a poroelastic 150x150 step).
-int grid_chain(int n, int ncomp) { return std::max(1, std::min((n + 255) / 256, 148 * (ncomp <= 2 ? 16 : 8))); }
+// Update of a chained step: up to 16 blocks an SM, twice the resident ones (the
+// blocks then end one after another and leave room for the next kernel's first
+// ones: fluid-solid 400x200 step 30.7 -> 28.8 us, SH 257x130 12.4 -> 12.2; no
+// difference for the poroelastic 150x150 step, 15.4 us).
+int grid_chain(int n) { return std::max(1, std::min((n + 255) / 256, 148 * 16)); }
 int grid_for(int n) {
   const int threads = 256;
   int blocks = (n + threads - 1) / threads;
@@ -845,7 +844,7 @@ void launch_update(sfg_handle *h, int medium, bool predict, bool advance, cudaSt
   const DevMedium &O = medium == SFG_MEDIUM_ELASTIC ? h->ac : h->el;
   sfg::dev::UpdateArgs U = update_args(h, D, O, medium, predict, advance);
   if (chained(h)) {
-    const int grid = grid_chain(U.n / D.ncomp, D.ncomp);
+    const int grid = grid_chain(U.n / D.ncomp);
     if (D.ncomp == 2) launch_pdl(sfg::dev::k_update_gather<2>, grid, 256, 0, s, U);
     else if (D.ncomp == 3) launch_pdl(sfg::dev::k_update_gather<3>, grid, 256, 0, s, U);
     else if (D.ncomp == 4) launch_pdl(sfg::dev::k_update_gather<4>, grid, 256, 0, s, U);
@@ -881,7 +880,7 @@ void launch_update_coupled(sfg_handle *h, bool predict, cudaStream_t s) {
   sfg::dev::UpdateArgs E = update_args(h, h->el, h->ac, SFG_MEDIUM_ELASTIC, predict, true);
   sfg::dev::UpdateArgs A = update_args(h, h->ac, h->el, SFG_MEDIUM_ACOUSTIC, predict, false);
   const int n = E.n / 2 + A.n - A.niface;
-  if (chained(h)) launch_pdl(sfg::dev::k_update_coupled, grid_chain(n, 2), 256, 0, s, E, A);
+  if (chained(h)) launch_pdl(sfg::dev::k_update_coupled, grid_chain(n), 256, 0, s, E, A);
   else sfg::dev::k_update_coupled<<<grid_for(n), 256, 0, s>>>(E, A);
 }
 
@@ -2838,10 +2837,10 @@ void reverse_segment_E(sfg_handle *h, int b, int n, bool last, cudaStream_t rs) 
       Ja.slot = i;
       launch_pdl(sfg::dev::k_adj_elem_ac<E>, ablocks, sfg::dev::NP * E, 0, rs, Ja);
       srcterm(C, Ac, i);
-      launch_pdl(sfg::dev::k_adj_post<2, true>, grid_for(D.nglob), 256, 0, rs,
+      launch_pdl(sfg::dev::k_adj_post<2, true>, grid_chain(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
           D.nglob, dt, dt2, dtsq2, cp_el);
-      launch_pdl(sfg::dev::k_adj_post<1, true>, grid_for(Ac.nglob), 256, 0, rs,
+      launch_pdl(sfg::dev::k_adj_post<1, true>, grid_chain(Ac.nglob), 256, 0, rs,
           C.lu, C.lv, C.mu, C.seg + 2 * C.nloc, C.seg_a + sl * C.stride, Ac.minv, C.r, Ac.inv_start,
           Ac.nglob, dt, dt2, dtsq2, cp_ac);
       psrc(C, Ac, i - 1);
@@ -2867,19 +2866,19 @@ void reverse_segment_E(sfg_handle *h, int b, int n, bool last, cudaStream_t rs) 
     if (A.pressure) {
       launch_pdl(sfg::dev::k_adj_elem_ac<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
       srcterm(A, D, i);
-      launch_pdl(sfg::dev::k_adj_post<1, false>, grid_for(D.nglob), 256, 0, rs,
+      launch_pdl(sfg::dev::k_adj_post<1, false>, grid_chain(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
           D.nglob, dt, dt2, dtsq2, sfg::dev::AdjCoupling{});
       psrc(A, D, i - 1);                      // mu of the previous step gets its source
     } else if (sh) {
       launch_pdl(sfg::dev::k_adj_elem_sh<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
-      launch_pdl(sfg::dev::k_adj_post<1, false>, grid_for(D.nglob), 256, 0, rs,
+      launch_pdl(sfg::dev::k_adj_post<1, false>, grid_chain(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
           D.nglob, dt, dt2, dtsq2, sfg::dev::AdjCoupling{});
     } else {
       if (ROW) row_elem(stacey);
       else launch_pdl(sfg::dev::k_adj_elem<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
-      launch_pdl(sfg::dev::k_adj_post<2, false>, grid_for(D.nglob), 256, 0, rs,
+      launch_pdl(sfg::dev::k_adj_post<2, false>, grid_chain(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
           D.nglob, dt, dt2, dtsq2, sfg::dev::AdjCoupling{});
     }
