@@ -52,7 +52,7 @@ typedef struct sfg_info3d {
   size_t device_bytes;
   int elements_per_block;
   int kernels_per_step;
-  int kernel_variant;           /* element-kernel form in use: 2 (column form) */
+  int kernel_variant;           /* element-kernel form in use: 2 (tiles marching in z) */
 } sfg_info3d;
 
 /* Reference: specfem::assembly::assembly<dim3> construction from the mesh. */

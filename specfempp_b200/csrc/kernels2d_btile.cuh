@@ -5,7 +5,7 @@
 // groups of four in the Morton order of the element centroids), sorted by
 // colour, and all the shots of a shot tile: one thread per element row (five
 // points) and quad of shots, the shots of a point across the lanes of a warp
-// as in k_stiffness_batched4r, whose element arithmetic this kernel repeats
+// as in the row form (k_stiffness_row), whose element arithmetic this kernel repeats
 // operation for operation.  The element results of the block are staged in
 // shared memory; a point that only the tile's elements touch (interior) is
 // then assembled in the block, its contributions summed in the tile's element
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(BT_E * NG * 8, 3) k_btile_row(BTileArgs P, int
   if (bad) *P.flag = 1;
 }
 
-// The points tiles share: k_update_batched4_gather over a list of points.
+// The points tiles share: k_update_batched_gather over a list of points.
 __global__ void __launch_bounds__(256) k_update_batched4_list(UpdateArgs A, int S, int NC, const int *pts, int npts) {
   const int per = NC * S / 4;   // quads per point
   const int n4 = npts * per;
