@@ -1486,6 +1486,7 @@ cudaGraphExec_t capture(sfg_handle *h, int nsteps, bool last_predicts) {
 // steps' graphs are captured when they are next used.
 void recapture(sfg_handle *h) {
   SFG_CUDA(cudaStreamSynchronize(h->stream));
+  if (h->adj.rstream) SFG_CUDA(cudaStreamSynchronize(h->adj.rstream));
   for (cudaGraphExec_t *g : {&h->graph_k, &h->graph_1, &h->graph_e, &h->graph_io, &h->adj.graph_r1, &h->adj.graph_re,
                              &h->adj.graph_rseg})
     if (*g) { cudaGraphExecDestroy(*g); *g = nullptr; }
@@ -2407,7 +2408,7 @@ int sfg_compute_seismograms(sfg_handle *h, int isig) {
 int sfg_set_model2d(sfg_handle *h, const float *rho, const float *kappa, const float *mu) {
   return guarded(h, [&]() {
     if (!rho || !kappa || !mu) return int(SFG_ERR_ARG);
-    const bool mat0 = row_matconst(h);
+    const bool el0 = h->asmb.el.row.matconst, ac0 = h->asmb.ac.row.matconst;
     sfg::set_model2d(h->mesh, h->asmb, rho, kappa, mu);
     // pressure sources in acoustic elements carry l / kappa: rebuild them
     const bool ac_src = h->have_sources && h->asmb.ac.nspec > 0 && h->asmb.nsrc > 0;
@@ -2428,8 +2429,9 @@ int sfg_set_model2d(sfg_handle *h, const float *rho, const float *kappa, const f
         put(D.minv, M.minv);
         put(D.erec, M.row.erec);
       }
-      // the step graphs hold the element kernels of the old model's class
-      if (row_matconst(h) != mat0) recapture(h);
+      // the graphs hold the element kernels of the old model's classes: the
+      // step's goes by both media together, the reverse sweep's by each
+      if (h->asmb.el.row.matconst != el0 || h->asmb.ac.row.matconst != ac0) recapture(h);
       refresh_tile_records(h);
       if (h->adj.st_c && !h->asmb.el.stacey_c.empty())
         SFG_CUDA(cudaMemcpy(h->adj.st_c, h->asmb.el.stacey_c.data(), h->asmb.el.stacey_c.size() * sizeof(float),

@@ -575,3 +575,46 @@ def test_coupled_adjoint_refusals(sfg_lib):
     sim2.initialize()
     with pytest.raises(sfg.SfgError, match="coupled adjoint"):
         sim2.forward_checkpointed(50, 10)
+
+
+# --------------------------------------------------------------------------
+# A handle that takes one model after another.
+
+
+def varied(model, where, seed):
+    """The model with +-5% at every point of the elements `where`."""
+    f = np.ones(model[0].shape)
+    f[where] = 1.0 + 0.05 * np.random.default_rng(seed).uniform(-1, 1, f[where].shape)
+    return [m * f for m in model]
+
+
+def test_coupled_gradient_after_each_medium_changes_class(sfg_lib):
+    """Row-form reverse sweep with several full segments: the water alone
+    varies inside its elements, then the solid alone, then the water again
+    (the pair of media is never constant as a whole).  Each gradient equals a
+    fresh handle's, bit for bit."""
+    from specfempp_b200 import sfg
+    n, interval = 160, 20
+    mesh, _, model, weights = coupled_problem("displacement", nstep=n)
+    water = np.asarray(mesh.mat_medium)[mesh.kmato] == 0
+
+    def handle():
+        sim = sfg.Simulation2D(mesh, dt=4e-4, nstep=n, kernel_variant=6)
+        sim.set_sources([sfg.Source(x=1500.0, z=1600.0, f0=25.0, factor=1e10),
+                         sfg.Source(x=900.0, z=1400.0, f0=25.0, factor=1e9, angle=30.0)])
+        sim.set_receivers(np.array([700.0, 900.0, 1500.0, 1800.0]), np.full(4, 1450.0), types=("displacement",))
+        sim.initialize()
+        return sim
+
+    def grad(sim, m):
+        sim.set_model(*[x.astype(np.float32) for x in m])
+        sim.forward_checkpointed(n, interval)
+        return sim.adjoint_gradient(weights)
+
+    models = [varied(model, water, 1), varied(model, ~water, 2), varied(model, water, 3)]
+    kept = handle()
+    for m in models:
+        got, want = grad(kept, m), grad(handle(), m)
+        for x, y in zip(got, want):
+            assert np.abs(y).max() > 0
+            assert np.array_equal(x, y)
