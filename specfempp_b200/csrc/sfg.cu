@@ -2433,9 +2433,14 @@ int sfg_set_model2d(sfg_handle *h, const float *rho, const float *kappa, const f
       // step's goes by both media together, the reverse sweep's by each
       if (h->asmb.el.row.matconst != el0 || h->asmb.ac.row.matconst != ac0) recapture(h);
       refresh_tile_records(h);
-      if (h->adj.st_c && !h->asmb.el.stacey_c.empty())
-        SFG_CUDA(cudaMemcpy(h->adj.st_c, h->asmb.el.stacey_c.data(), h->asmb.el.stacey_c.size() * sizeof(float),
-                            cudaMemcpyHostToDevice));
+      // the sweep's absorbing points: adj is the elastic medium, or the only
+      // one; adj2 the acoustic medium of a coupled model
+      const std::vector<float> &c1 = h->el.nspec ? h->asmb.el.stacey_c : h->asmb.ac.stacey_c;
+      const std::vector<float> &c2 = h->asmb.ac.stacey_c;
+      if (h->adj.st_c && !c1.empty())
+        SFG_CUDA(cudaMemcpy(h->adj.st_c, c1.data(), c1.size() * sizeof(float), cudaMemcpyHostToDevice));
+      if (h->adj2.st_c && !c2.empty())
+        SFG_CUDA(cudaMemcpy(h->adj2.st_c, c2.data(), c2.size() * sizeof(float), cudaMemcpyHostToDevice));
       h->adj.forward_done = false;
     }
     return int(SFG_OK);

@@ -618,3 +618,33 @@ def test_coupled_gradient_after_each_medium_changes_class(sfg_lib):
         for x, y in zip(got, want):
             assert np.abs(y).max() > 0
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("kind", ["acoustic", "coupled"])
+def test_absorbing_water_edges_follow_the_model(sfg_lib, kind):
+    """The sweep's impedances of the acoustic medium's absorbing points belong
+    to the model of the gradient: a second model's gradient equals a fresh
+    handle's, bit for bit.  The acoustic source is 700 m from an edge."""
+    def fresh():
+        if kind == "acoustic":
+            (sx, sz), _, _, nstep, rz = ACOUSTIC_CASES["absorbing_edge"]
+            w, sim, model, weights = acoustic_problem(sx, sz, nstep, rz)
+            return w.mesh, sim, model, weights
+        return coupled_problem("pressure", nstep=NSTEP)
+
+    mesh, kept, model, weights = fresh()
+    water = np.asarray(mesh.mat_medium)[mesh.kmato] == 0
+    second = [m.copy() for m in model]
+    second[0][water] *= 1.1
+    second[1][water] *= 1.3
+
+    def grad(sim, m):
+        sim.set_model(*[x.astype(np.float32) for x in m])
+        sim.forward_checkpointed(len(weights), 50)
+        return sim.adjoint_gradient(weights)
+
+    grad(kept, model)
+    got, want = grad(kept, second), grad(fresh()[1], second)
+    for x, y in zip(got, want):
+        assert np.abs(y).max() > 0
+        assert np.array_equal(x, y)
