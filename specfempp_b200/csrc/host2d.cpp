@@ -763,13 +763,13 @@ void classify_rows(MediumData &D) {
 
 void set_model2d(Mesh2D &m, Assembly2D &a, const float *rho, const float *kappa, const float *mu) {
   const size_t n = size_t(m.nspec) * NPTS;
-  m.prho.resize(n);
-  m.pvp.resize(n);
-  m.pvs.resize(n);
   bool bad = false;
 #pragma omp parallel for schedule(static) reduction(|| : bad)
   for (size_t p = 0; p < n; ++p) bad = bad || !(rho[p] > 0) || !(mu[p] >= 0) || !(kappa[p] + 4.0 / 3.0 * mu[p] > 0);
   if (bad) throw std::runtime_error("model values must give rho > 0, mu >= 0, lambda + 2 mu > 0");
+  m.prho.resize(n);
+  m.pvp.resize(n);
+  m.pvs.resize(n);
 #pragma omp parallel for schedule(static)
   for (size_t p = 0; p < n; ++p) {
     m.prho[p] = rho[p];

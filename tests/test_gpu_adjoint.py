@@ -648,3 +648,28 @@ def test_absorbing_water_edges_follow_the_model(sfg_lib, kind):
     for x, y in zip(got, want):
         assert np.abs(y).max() > 0
         assert np.array_equal(x, y)
+
+
+def test_refused_model_leaves_the_handle_as_it_was(sfg_lib):
+    """A model with a non-positive density is refused; the next gradient is
+    that of the materials the handle was made with, absorbing edges
+    included."""
+    from specfempp_b200 import meshgen, sfg
+    w = meshgen.elastic_psv_80x60(nstep=200)
+    rng = np.random.default_rng(5)
+    weights = rng.standard_normal((200, 1, 2)).astype(np.float32)
+    out = []
+    for refused in (False, True):
+        sim = sfg.Simulation2D(w.mesh, dt=w.dt, nstep=200)
+        sim.set_sources([sfg.Source(x=150.0, z=1500.0, f0=30.0, factor=1e10)])
+        sim.set_receivers(np.array([200.0]), np.array([1550.0]), types=("displacement",))
+        sim.initialize()
+        if refused:
+            bad = [m.astype(np.float32) for m in base_model(w.mesh)]
+            bad[0][7, 3] = 0.0
+            with pytest.raises(sfg.SfgError, match="rho > 0"):
+                sim.set_model(*bad)
+        sim.forward_checkpointed(200, 50)
+        out.append(sim.adjoint_gradient(weights))
+    for x, y in zip(*out):
+        assert np.abs(x).max() > 0 and np.array_equal(x, y)
