@@ -904,9 +904,15 @@ int sfg3d_step_io(sfg_handle3d *h, const float *stf_row, float *seis_row) {
 int sfg3d_time_kernel(sfg_handle3d *h, int which, int reps, float *ms) {
   return guarded(h, [&]() {
     if (!h->initialized || !ms || reps <= 0) return int(SFG_ERR_ARG);
-    // the launches read the fields' buffers and write the other pair, which
-    // the next step overwrites: the state is as before
-    const sfg3::dev::Step3Args A = step_args(h, true, false);
+    // The launches read the fields' buffers and write the other pair, which
+    // the next step overwrites, and step[1], which its layer kernel sets; the
+    // acceleration and the flag go to scratch, and receivers store nothing.
+    sfg3::DevMem scratch;
+    sfg3::dev::Step3Args A = step_args(h, true, false);
+    if (A.a_store) A.a_store = scratch.zeros<float>(size_t(h->nglob) * 3 + 4);
+    A.flag = scratch.zeros<int>(1);
+    A.nsig = 0;
+    SFG3_CUDA(cudaDeviceSynchronize());
     SFG3_CUDA(cudaEventRecord(h->ev0, h->stream));
     for (int i = 0; i < reps; ++i) {
       if (which == 0) launch_layers(h, A, h->stream);

@@ -147,3 +147,45 @@ def test_specfem3d_config_driver(sfg_lib, oracle_lib, tmp_path):
         assert err.max() < 1e-3, (kind, err.max())
         # the files hold 7 significant digits (%e), well inside the bar
         assert rel_l2(np.transpose(got, (2, 0, 1)), ref[:, t]) <= tol(kind), kind
+
+
+def small_handle(nstep=60, epb=0, types=("displacement",), shape=(5, 3, 4)):
+    """An initialised handle of a small mesh of boxes with Stacey sides."""
+    from oracle import runner3d
+    from specfempp_b200 import meshgen, sfg3d
+    nx, ny, nz = shape
+    m = meshgen.homogeneous_hex_mesh(nx, ny, nz, (0, 60.0 * nx, 0, 50.0 * ny, -55.0 * nz, 0), 2300.0, 3000.0, 1700.0,
+                                     absorbing=(1, 0, 1, 1, 1, 0))
+    W, D, H = 60.0 * nx, 50.0 * ny, 55.0 * nz
+    sim = sfg3d.Simulation3D(m, dt=3e-4, nstep=nstep, elements_per_block=epb)
+    sim.set_sources([runner3d.Source3D(0.6 * W, 0.4 * D, -0.6 * H, f0=60.0, factor=1e10, comp=(0.2, 1.0, -0.6, 0, 0, 0))])
+    sim.set_receivers(np.array([[0.5 * W, 0.45 * D, -0.55 * H], [0.7 * W, 0.6 * D, -0.65 * H]]), types=types)
+    sim.initialize()
+    return sim
+
+
+@pytest.mark.parametrize("types", [("displacement",), ("velocity",), ("displacement", "acceleration")])
+def test_3d_timing_a_kernel_leaves_the_run_alone(sfg_lib, types):
+    """Both kernels timed after a run and after a streamed step: fields,
+    seismograms and the rest of the run are those of an untimed handle."""
+    a, b = small_handle(types=types), small_handle(types=types)
+    row = np.zeros((len(types), 2, 3), np.float32)
+
+    def timed():
+        assert b.time_kernel(0, 3) > 0 and b.time_kernel(1, 3) > 0
+
+    for s in (a, b):
+        s.run(40)
+    timed()
+    for f in ("displacement", "velocity", "acceleration"):
+        assert np.array_equal(a.field(f), b.field(f)), f
+    assert np.abs(a.field("acceleration")).max() > 0
+    for s in (a, b):
+        s.step_io(None, row)
+    timed()
+    assert np.array_equal(a.seismograms(), b.seismograms())
+    for s in (a, b):
+        s.run(19)
+    assert np.array_equal(a.seismograms(), b.seismograms())
+    assert np.array_equal(a.field("displacement"), b.field("displacement"))
+    assert a.check_finite() and b.check_finite()
