@@ -213,6 +213,7 @@ struct sfg_handle {
   // receivers the next element launch takes (set around it by enqueue_step)
   sfg::dev::RecArgs *d_rec_args = nullptr;
   bool early_now[2] = {false, false};
+  bool timing = false;             // sfg_time_kernel: launches one after another
   int *d_rec_elem = nullptr;
   float *d_rec_h = nullptr, *d_seis = nullptr;
   int *d_step = nullptr, *d_flag = nullptr;
@@ -395,9 +396,12 @@ int ncolors(const DevMedium &D) { return D.nspec ? int(D.color_start.size()) - 1
 
 // Launch as a programmatic dependent of the kernel before it on the stream
 // (pdl_wait in kernels2d.cuh): only for kernels that call pdl_wait on every
-// thread before they touch data of the step.
+// thread before they touch data of the step, and only after a kernel that
+// writes nothing that this one reads before that wait.  The updates read their
+// own u and v there, so none follows an update of its own medium this way;
+// sfg_time_kernel, which repeats one kernel, launches without the attribute.
 template <typename... P, typename... A>
-void launch_pdl(void (*kern)(P...), int grid, int block, size_t smem, cudaStream_t s, A &&...args) {
+void launch_pdl(const sfg_handle *h, void (*kern)(P...), int grid, int block, size_t smem, cudaStream_t s, A &&...args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(unsigned(grid));
   cfg.blockDim = dim3(unsigned(block));
@@ -405,7 +409,7 @@ void launch_pdl(void (*kern)(P...), int grid, int block, size_t smem, cudaStream
   cfg.stream = s;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+  at.val.programmaticStreamSerializationAllowed = h->timing ? 0 : 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   SFG_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
@@ -459,7 +463,7 @@ void launch_stiffness_E(sfg_handle *h, const DevMedium &el, const DevMedium &ac,
     S.ac.e0 = 0; S.ac.e1 = ac.nspec; S.ac.nblocks = (ac.nspec + E - 1) / E;
     early_receivers(h, S, sfg::dev::NP * E, h->early_now[0], h->early_now[1]);
     const int grid = S.el.nblocks + S.ac.nblocks + S.rec_blocks + S.save_blocks;
-    if (grid > 0) launch_pdl(sfg::dev::k_stiffness<E, EK, true>, grid, sfg::dev::NP * E, 0, s, S);
+    if (grid > 0) launch_pdl(h, sfg::dev::k_stiffness<E, EK, true>, grid, sfg::dev::NP * E, 0, s, S);
     return;
   }
   if (variant == 4) {
@@ -662,7 +666,7 @@ void launch_stiffness_row(sfg_handle *h, const DevMedium &el, const DevMedium &a
   if (grid == 0) return;
   if (!S.el.erec && !S.ac.erec) throw std::runtime_error("row-form element kernel: element records missing on the device");
   const int geo = row_straight(h) ? 1 : 0, mat = row_matconst(h) ? 1 : 0;
-  auto go = [&](auto kern) { launch_pdl(kern, grid, sfg::dev::NG * E, 0, s, S); };
+  auto go = [&](auto kern) { launch_pdl(h, kern, grid, sfg::dev::NG * E, 0, s, S); };
   if (el.nspec && el.ncomp == 4) {
     if (geo) go(sfg::dev::k_stiffness_row<E, 4, 1, 1>);
     else go(sfg::dev::k_stiffness_row<E, 4, 0, 1>);
@@ -835,7 +839,7 @@ void launch_receivers(sfg_handle *h, int medium, cudaStream_t s) {
   if (D.nrec == 0) return;
   const sfg::dev::RecArgs R = rec_args(h, medium);
   if (D.S > 1) sfg::dev::k_receivers_batched<<<D.nrec, 32, 0, s>>>(R, D.S);
-  else if (chained(h)) launch_pdl(sfg::dev::k_receivers, D.nrec, 32, 0, s, R);
+  else if (chained(h)) launch_pdl(h, sfg::dev::k_receivers, D.nrec, 32, 0, s, R);
   else sfg::dev::k_receivers<<<D.nrec, 32, 0, s>>>(R);
 }
 
@@ -845,10 +849,10 @@ void launch_update(sfg_handle *h, int medium, bool predict, bool advance, cudaSt
   sfg::dev::UpdateArgs U = update_args(h, D, O, medium, predict, advance);
   if (chained(h)) {
     const int grid = grid_chain(U.n / D.ncomp);
-    if (D.ncomp == 2) launch_pdl(sfg::dev::k_update_gather<2>, grid, 256, 0, s, U);
-    else if (D.ncomp == 3) launch_pdl(sfg::dev::k_update_gather<3>, grid, 256, 0, s, U);
-    else if (D.ncomp == 4) launch_pdl(sfg::dev::k_update_gather<4>, grid, 256, 0, s, U);
-    else launch_pdl(sfg::dev::k_update_gather<1>, grid, 256, 0, s, U);
+    if (D.ncomp == 2) launch_pdl(h, sfg::dev::k_update_gather<2>, grid, 256, 0, s, U);
+    else if (D.ncomp == 3) launch_pdl(h, sfg::dev::k_update_gather<3>, grid, 256, 0, s, U);
+    else if (D.ncomp == 4) launch_pdl(h, sfg::dev::k_update_gather<4>, grid, 256, 0, s, U);
+    else launch_pdl(h, sfg::dev::k_update_gather<1>, grid, 256, 0, s, U);
     return;
   }
   if (h->variant >= 3) {
@@ -880,7 +884,7 @@ void launch_update_coupled(sfg_handle *h, bool predict, cudaStream_t s) {
   sfg::dev::UpdateArgs E = update_args(h, h->el, h->ac, SFG_MEDIUM_ELASTIC, predict, true);
   sfg::dev::UpdateArgs A = update_args(h, h->ac, h->el, SFG_MEDIUM_ACOUSTIC, predict, false);
   const int n = E.n / 2 + A.n - A.niface;
-  if (chained(h)) launch_pdl(sfg::dev::k_update_coupled, grid_chain(n), 256, 0, s, E, A);
+  if (chained(h)) launch_pdl(h, sfg::dev::k_update_coupled, grid_chain(n), 256, 0, s, E, A);
   else sfg::dev::k_update_coupled<<<grid_for(n), 256, 0, s>>>(E, A);
 }
 
@@ -2124,6 +2128,11 @@ int sfg_time_kernel_flushed(sfg_handle *h, int which, int iters, size_t flush_by
       else launch_update(h, medium, true, false, h->stream);
     };
     h->state_final = false;
+    struct Timing {
+      bool &on;
+      explicit Timing(bool &b) : on(b) { on = true; }
+      ~Timing() { on = false; }
+    } alone(h->timing);
     for (int i = 0; i < 3; ++i) launch();
     float t = 0;
     if (flush_bytes == 0) {
@@ -2790,12 +2799,12 @@ void reverse_segment_E(sfg_handle *h, int b, int n, bool last, cudaStream_t rs) 
   const size_t ob = size_t(b) * A.interval;
   auto psrc = [&](AdjointState &X, const DevMedium &M, int slot) {
     if (X.nps)
-      launch_pdl(sfg::dev::k_adj_psrc, std::min(grid_for(X.nps), 64), 128, 0, rs,
+      launch_pdl(h, sfg::dev::k_adj_psrc, std::min(grid_for(X.nps), 64), 128, 0, rs,
           X.mu, M.minv, X.ps_pt, X.ps_start, X.ps_rec, X.ps_h, A.gtab, A.d_k0, slot, h->asmb.nrec, X.nps);
   };
   auto srcterm = [&](AdjointState &X, const DevMedium &M, int slot) {
     if (X.nsrc_t)
-      launch_pdl(sfg::dev::k_adj_srcterm, (X.nsrc_t * sfg::NPTS + 127) / 128, 128, 0, rs,
+      launch_pdl(h, sfg::dev::k_adj_srcterm, (X.nsrc_t * sfg::NPTS + 127) / 128, 128, 0, rs,
           X.seg + X.off_src(), X.mu, M.ibool, X.src_ce, h->d_stf, A.d_k0, slot, X.nsrc_t, h->asmb.nstep,
           X.src_id, h->asmb.nsrc);
   };
@@ -2804,7 +2813,7 @@ void reverse_segment_E(sfg_handle *h, int b, int n, bool last, cudaStream_t rs) 
     const int sb = stacey ? St.nb_grad + grid_for(A.nst) : 0;
     const bool geo = h->asmb.el.row.straight, mat = h->asmb.el.row.matconst;
     auto go = [&](auto kern) {
-      launch_pdl(kern, (D.nspec + 31) / 32 + sb, sfg::dev::NG * 32, 0, rs, J, med_args(D), St, sb);
+      launch_pdl(h, kern, (D.nspec + 31) / 32 + sb, sfg::dev::NG * 32, 0, rs, J, med_args(D), St, sb);
     };
     if (geo && mat) go(sfg::dev::k_adj_elem_row<32, 1, 1>);
     else if (geo) go(sfg::dev::k_adj_elem_row<32, 1, 0>);
@@ -2829,25 +2838,25 @@ void reverse_segment_E(sfg_handle *h, int b, int n, bool last, cudaStream_t rs) 
       if (A.nst) {
         St.vst = A.seg_v + sl * A.vstride;
         St.af = A.seg_a + sl * A.stride;
-        if (!ROW) launch_pdl(sfg::dev::k_adj_stacey<2>, St.nb_grad + grid_for(A.nst), 256, 0, rs, St);
+        if (!ROW) launch_pdl(h, sfg::dev::k_adj_stacey<2>, St.nb_grad + grid_for(A.nst), 256, 0, rs, St);
       }
       if (C.nst) {
         Sa.vst = C.seg_v + sl * C.vstride;
         Sa.af = C.seg_a + sl * C.stride;
-        launch_pdl(sfg::dev::k_adj_stacey<1>, Sa.nb_grad + grid_for(C.nst), 256, 0, rs, Sa);
+        launch_pdl(h, sfg::dev::k_adj_stacey<1>, Sa.nb_grad + grid_for(C.nst), 256, 0, rs, Sa);
       }
       J.uf = A.seg_u + sl * A.stride;
       J.slot = i;
       if (ROW) row_elem(A.nst > 0);
-      else launch_pdl(sfg::dev::k_adj_elem<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
+      else launch_pdl(h, sfg::dev::k_adj_elem<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
       Ja.uf = C.seg_u + sl * C.stride;
       Ja.slot = i;
-      launch_pdl(sfg::dev::k_adj_elem_ac<E>, ablocks, sfg::dev::NP * E, 0, rs, Ja);
+      launch_pdl(h, sfg::dev::k_adj_elem_ac<E>, ablocks, sfg::dev::NP * E, 0, rs, Ja);
       srcterm(C, Ac, i);
-      launch_pdl(sfg::dev::k_adj_post<2, true>, grid_chain(D.nglob), 256, 0, rs,
+      launch_pdl(h, sfg::dev::k_adj_post<2, true>, grid_chain(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
           D.nglob, dt, dt2, dtsq2, cp_el);
-      launch_pdl(sfg::dev::k_adj_post<1, true>, grid_chain(Ac.nglob), 256, 0, rs,
+      launch_pdl(h, sfg::dev::k_adj_post<1, true>, grid_chain(Ac.nglob), 256, 0, rs,
           C.lu, C.lv, C.mu, C.seg + 2 * C.nloc, C.seg_a + sl * C.stride, Ac.minv, C.r, Ac.inv_start,
           Ac.nglob, dt, dt2, dtsq2, cp_ac);
       psrc(C, Ac, i - 1);
@@ -2865,27 +2874,27 @@ void reverse_segment_E(sfg_handle *h, int b, int n, bool last, cudaStream_t rs) 
       St.vst = A.seg_v + sl * A.vstride;
       St.af = A.seg_a + sl * A.stride;
       if (ROW) {}      // in the element launch
-      else if (sh) launch_pdl(sfg::dev::k_adj_stacey<1>, St.nb_grad + grid_for(A.nst), 256, 0, rs, St);
-      else launch_pdl(sfg::dev::k_adj_stacey<2>, St.nb_grad + grid_for(A.nst), 256, 0, rs, St);
+      else if (sh) launch_pdl(h, sfg::dev::k_adj_stacey<1>, St.nb_grad + grid_for(A.nst), 256, 0, rs, St);
+      else launch_pdl(h, sfg::dev::k_adj_stacey<2>, St.nb_grad + grid_for(A.nst), 256, 0, rs, St);
     }
     J.uf = A.seg_u + sl * A.stride;
     J.slot = i;
     if (A.pressure) {
-      launch_pdl(sfg::dev::k_adj_elem_ac<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
+      launch_pdl(h, sfg::dev::k_adj_elem_ac<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
       srcterm(A, D, i);
-      launch_pdl(sfg::dev::k_adj_post<1, false>, grid_chain(D.nglob), 256, 0, rs,
+      launch_pdl(h, sfg::dev::k_adj_post<1, false>, grid_chain(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
           D.nglob, dt, dt2, dtsq2, sfg::dev::AdjCoupling{});
       psrc(A, D, i - 1);                      // mu of the previous step gets its source
     } else if (sh) {
-      launch_pdl(sfg::dev::k_adj_elem_sh<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
-      launch_pdl(sfg::dev::k_adj_post<1, false>, grid_chain(D.nglob), 256, 0, rs,
+      launch_pdl(h, sfg::dev::k_adj_elem_sh<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
+      launch_pdl(h, sfg::dev::k_adj_post<1, false>, grid_chain(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
           D.nglob, dt, dt2, dtsq2, sfg::dev::AdjCoupling{});
     } else {
       if (ROW) row_elem(stacey);
-      else launch_pdl(sfg::dev::k_adj_elem<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
-      launch_pdl(sfg::dev::k_adj_post<2, false>, grid_chain(D.nglob), 256, 0, rs,
+      else launch_pdl(h, sfg::dev::k_adj_elem<E>, eblocks, sfg::dev::NP * E, 0, rs, J);
+      launch_pdl(h, sfg::dev::k_adj_post<2, false>, grid_chain(D.nglob), 256, 0, rs,
           A.lu, A.lv, A.mu, A.seg + 2 * A.nloc, A.seg_a + sl * A.stride, D.minv, A.r, D.inv_start,
           D.nglob, dt, dt2, dtsq2, sfg::dev::AdjCoupling{});
     }

@@ -472,7 +472,7 @@ void setup_sources(sfg_handle3d *h) {
 bool valid_layers(int e) { return e == 1 || e == 2 || e == 4 || e == 6 || e == 8; }
 
 template <typename... P, typename... A>
-void launch_pdl(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A &&...args) {
+void launch_pdl(bool dependent, void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A &&...args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(unsigned(block));
@@ -480,7 +480,7 @@ void launch_pdl(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStrea
   cfg.stream = s;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+  at.val.programmaticStreamSerializationAllowed = dependent ? 1 : 0;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   SFG3_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
@@ -498,15 +498,15 @@ sfg3::dev::Step3Args step_args(const sfg_handle3d *h, bool predict, bool advance
   return A;
 }
 
-void launch_layers(const sfg_handle3d *h, const sfg3::dev::Step3Args &A, cudaStream_t s) {
+void launch_layers(const sfg_handle3d *h, const sfg3::dev::Step3Args &A, cudaStream_t s, bool dependent = true) {
   const dim3 grid(unsigned(A.nbx * A.nby), unsigned(A.nchunk));
-  if (h->boxes) launch_pdl(sfg3::dev::k_layer3d<1>, grid, sfg3::dev::TILE_THREADS, sfg3::dev::L3_SMEM, s, A);
-  else launch_pdl(sfg3::dev::k_layer3d<0>, grid, sfg3::dev::TILE_THREADS, sfg3::dev::L3_SMEM, s, A);
+  if (h->boxes) launch_pdl(dependent, sfg3::dev::k_layer3d<1>, grid, sfg3::dev::TILE_THREADS, sfg3::dev::L3_SMEM, s, A);
+  else launch_pdl(dependent, sfg3::dev::k_layer3d<0>, grid, sfg3::dev::TILE_THREADS, sfg3::dev::L3_SMEM, s, A);
 }
 
-void launch_finish(const sfg3::dev::Step3Args &A, cudaStream_t s) {
+void launch_finish(const sfg3::dev::Step3Args &A, cudaStream_t s, bool dependent = true) {
   const int ntile = A.nbx * A.nby, planes = sfg3::dev::finish_planes(ntile, A.NZ), ngroup = (A.NZ + planes - 1) / planes;
-  launch_pdl(sfg3::dev::k_finish3d, dim3(unsigned(A.rec_blocks + ntile * (ngroup + A.nchunk - 1))), 256, 0, s, A);
+  launch_pdl(dependent, sfg3::dev::k_finish3d, dim3(unsigned(A.rec_blocks + ntile * (ngroup + A.nchunk - 1))), 256, 0, s, A);
 }
 
 // One step from buffer par into the other; par flips.
@@ -514,7 +514,7 @@ void launch_step(sfg_handle3d *h, cudaStream_t s, bool predict) {
   const sfg3::dev::Step3Args A = step_args(h, predict, true);
   launch_layers(h, A, s);
   launch_finish(A, s);
-  if (h->late) launch_pdl(sfg3::dev::k_receivers3d, dim3(unsigned(h->nrec)), 128, 0, s, A);
+  if (h->late) launch_pdl(true, sfg3::dev::k_receivers3d, dim3(unsigned(h->nrec)), 128, 0, s, A);
   h->par ^= 1;
 }
 
@@ -915,8 +915,8 @@ int sfg3d_time_kernel(sfg_handle3d *h, int which, int reps, float *ms) {
     SFG3_CUDA(cudaDeviceSynchronize());
     SFG3_CUDA(cudaEventRecord(h->ev0, h->stream));
     for (int i = 0; i < reps; ++i) {
-      if (which == 0) launch_layers(h, A, h->stream);
-      else launch_finish(A, h->stream);
+      if (which == 0) launch_layers(h, A, h->stream, false);
+      else launch_finish(A, h->stream, false);
     }
     SFG3_CUDA(cudaEventRecord(h->ev1, h->stream));
     SFG3_CUDA(cudaEventSynchronize(h->ev1));

@@ -193,3 +193,22 @@ def test_3d_tiles_against_the_oracle(sfg_lib, oracle_lib, shape, relief):
     assert rel_l2(first[1], ref["final"]) <= 1e-5
     for t in range(2):
         assert rel_l2(first[0][:, t], ref["seis"][:, t]) <= 1e-5
+
+
+@pytest.mark.parametrize("kind", ["psv", "sh", "acoustic", "poro"])
+def test_timed_point_updates_run_one_after_another(sfg_lib, kind):
+    """sfg_time_kernel repeats the point update, which reads the fields that
+    the update before it wrote: the state afterwards, and a step from it, are
+    the same bits for every form of the step (4, which has no chained
+    launches, where the medium has it)."""
+    med, which = ("acoustic", 2) if kind == "acoustic" else ("elastic", 1)
+    fields = []
+    for v in ((3, 6) if kind == "poro" else (4, 3, 6)):
+        sim = simulate(grid(kind, 45, 31, 0.0), kind, 60, v, 16)
+        assert sim.info().kernel_variant == v
+        assert sim.time_kernel(which, 20) > 0
+        sim.run(1)
+        fields.append((sim.field(med), sim.field(med, "velocity")))
+    assert np.abs(fields[0][0]).max() > 0
+    for f in fields[1:]:
+        assert np.array_equal(f[0], fields[0][0]) and np.array_equal(f[1], fields[0][1])
