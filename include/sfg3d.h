@@ -5,8 +5,9 @@
  * media given per GLL point, force and moment-tensor sources, receivers, the
  * Newmark time loop captured in CUDA graphs.  Status codes and sfg_options
  * are those of sfg.h (elements_per_block, 1, 2, 4, 6 or 8, fixes the layers of
- * elements that a block of the layer kernel marches through; 0 lets the
- * autotuner choose; all give the same bits; kernel_variant is ignored).
+ * elements that a block of the layer kernel marches through, or the least that
+ * needs no more than 65,535 blocks in z; 0 lets the autotuner choose; all give
+ * the same bits; kernel_variant is ignored).
  *
  * It replaces, for this mesh class, the reference's dim3 forward path:
  * the assembly (core/specfem/assembly/ dim3 containers), the element kernel

@@ -762,11 +762,14 @@ int sfg3d_initialize(sfg_handle3d *h) {
     SFG3_CUDA(cudaFuncSetAttribute(sfg3::dev::k_layer3d<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    sfg3::dev::L3_SMEM));
     // the tiles' parts of shared points: sized for the shortest march tried
+    // (the grid's second dimension holds at most 65,535 of them)
+    const int least = (h->nez + 65534) / 65535;
     std::vector<int> cand;
-    if (valid_layers(h->opt.elements_per_block)) cand = {h->opt.elements_per_block};
+    if (valid_layers(h->opt.elements_per_block)) cand = {std::max(h->opt.elements_per_block, least)};
     else
       for (int L : {1, 2, 4, 8, 16})
-        if (L == 1 || L < 2 * h->nez) cand.push_back(L);
+        if (L >= least && (L == 1 || L < 2 * h->nez)) cand.push_back(L);
+    if (cand.empty()) cand.push_back(least);
     const size_t ntile = size_t(A.nbx) * A.nby;
     A.rim = m.zeros<float>(ntile * A.NZ * sfg3::dev::NEDGE * 3);
     const size_t parts = ntile * size_t((h->nez + cand[0] - 1) / cand[0]) * sfg3::dev::NCOL * 3;

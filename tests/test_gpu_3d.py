@@ -189,3 +189,16 @@ def test_3d_timing_a_kernel_leaves_the_run_alone(sfg_lib, types):
     assert np.array_equal(a.seismograms(), b.seismograms())
     assert np.array_equal(a.field("displacement"), b.field("displacement"))
     assert a.check_finite() and b.check_finite()
+
+
+@pytest.mark.parametrize("epb", [1, 0])
+def test_3d_more_layers_than_a_grid_dimension(sfg_lib, epb):
+    """A column of 65,540 elements: one block a layer is above 65,535 blocks.
+    The same bits as eight layers a block."""
+    shape = (1, 1, 65540)
+    a = small_handle(nstep=3, epb=8, shape=shape)
+    b = small_handle(nstep=3, epb=epb, shape=shape)
+    for s in (a, b):
+        s.run(3)
+    u = a.field("displacement")
+    assert np.abs(u).max() > 0 and np.array_equal(u, b.field("displacement"))
