@@ -300,12 +300,34 @@ int guarded(sfg_handle *h, F &&fn) {
   try {
     return fn();
   } catch (const CudaError &ex) {
+    cudaGetLastError();       // reported here, not by the next handle's call
     h->err = ex.what();
     return SFG_ERR_CUDA;
   } catch (const std::exception &ex) {
     h->err = ex.what();
     return SFG_ERR_ARG;
   }
+}
+
+// Graph of what `work` launches on s.  A launch that is refused ends the
+// capture too: while one is open, the thread may not allocate.
+template <typename F>
+cudaGraphExec_t capture_graph(cudaStream_t s, F &&work) {
+  cudaGraph_t g = nullptr;
+  SFG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+  try {
+    work();
+    SFG_CUDA(cudaGetLastError());
+  } catch (...) {
+    if (cudaStreamEndCapture(s, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+    throw;
+  }
+  SFG_CUDA(cudaStreamEndCapture(s, &g));
+  cudaGraphExec_t ex = nullptr;
+  const cudaError_t rc = cudaGraphInstantiate(&ex, g, 0);
+  cudaGraphDestroy(g);
+  SFG_CUDA(rc);
+  return ex;
 }
 
 void upload_medium(sfg_handle *h, const sfg::MediumData &M, DevMedium &D) {
@@ -1476,14 +1498,9 @@ bool fused_update(const sfg_handle *h) {
 }
 
 cudaGraphExec_t capture(sfg_handle *h, int nsteps, bool last_predicts) {
-  cudaGraph_t g = nullptr;
-  SFG_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  for (int i = 0; i < nsteps; ++i) enqueue_step(h, h->stream, i + 1 < nsteps || last_predicts);
-  SFG_CUDA(cudaStreamEndCapture(h->stream, &g));
-  cudaGraphExec_t ex = nullptr;
-  SFG_CUDA(cudaGraphInstantiate(&ex, g, 0));
-  cudaGraphDestroy(g);
-  return ex;
+  return capture_graph(h->stream, [&]() {
+    for (int i = 0; i < nsteps; ++i) enqueue_step(h, h->stream, i + 1 < nsteps || last_predicts);
+  });
 }
 
 // Capture the step graphs (again); the streamed, the recording and the reverse
@@ -2064,16 +2081,13 @@ int sfg_step_io(sfg_handle *h, const float *stf_row, float *seis_row) {
       // one fused step (the next step's predictor applied in the update)
       // between the row copies; the step's seismograms are complete before
       // its update runs
-      cudaGraph_t g = nullptr;
-      SFG_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-      k_io_in<<<1, 128, 0, h->stream>>>(io_d, h->d_stf, h->d_step, a.nsrc, a.nstep);
-      enqueue_step(h, h->stream, true);
-      if (a.nrec > 0)
-        k_io_out<<<std::max(1, std::min(64, (a.nshots * rowlen + 255) / 256)), 256, 0, h->stream>>>(
-            h->d_seis, seis_d, h->d_step, a.nsb, a.nsig, a.nshots, rowlen);
-      SFG_CUDA(cudaStreamEndCapture(h->stream, &g));
-      SFG_CUDA(cudaGraphInstantiate(&h->graph_io, g, 0));
-      cudaGraphDestroy(g);
+      h->graph_io = capture_graph(h->stream, [&]() {
+        k_io_in<<<1, 128, 0, h->stream>>>(io_d, h->d_stf, h->d_step, a.nsrc, a.nstep);
+        enqueue_step(h, h->stream, true);
+        if (a.nrec > 0)
+          k_io_out<<<std::max(1, std::min(64, (a.nshots * rowlen + 255) / 256)), 256, 0, h->stream>>>(
+              h->d_seis, seis_d, h->d_step, a.nsb, a.nsig, a.nshots, rowlen);
+      });
     }
     int *io = static_cast<int *>(h->io_host);
     io[0] = 0;
@@ -2699,19 +2713,21 @@ void adjoint_alloc(sfg_handle *h, int nstep, int interval) {
   if (cpl && !A2.lu) adj_medium_init(h, A2, h->ac, h->asmb.ac, SFG_MEDIUM_ACOUSTIC);
   adj_write_record(A, D);
   if (cpl) adj_write_record(A2, h->ac);
+  auto recorded = [&](int mode, int nsteps, bool last_predicts) {
+    struct Off {
+      int &mode;
+      ~Off() { mode = 0; }
+    } off{h->recording};
+    h->recording = mode;
+    return capture(h, nsteps, last_predicts);
+  };
   if (!A.graph_r1) {
     // one recording step with the next predictor fused, and one ending on
     // the corrector (the segment's last step)
-    h->recording = 1;
-    A.graph_r1 = capture(h, 1, true);
-    A.graph_re = capture(h, 1, false);
-    h->recording = 0;
+    A.graph_r1 = recorded(1, 1, true);
+    A.graph_re = recorded(1, 1, false);
   }
-  if (!A.graph_rseg && interval > 1) {
-    h->recording = 2;
-    A.graph_rseg = capture(h, interval - 1, true);
-    h->recording = 0;
-  }
+  if (!A.graph_rseg && interval > 1) A.graph_rseg = recorded(2, interval - 1, true);
 }
 
 // Checkpoint c of every medium in the sweep: u, v, a at the segment's start.
@@ -3073,14 +3089,8 @@ int sfg_adjoint_gradient(sfg_handle *h, const float *seis_grad, float *grad_rho,
       sfg::dev::k_set_step<<<1, 1, 0, rs>>>(A.d_k0, k0);
       if (c + 1 < A.ncheck && k1 - k0 == A.interval) {
         // full segment, not the run's last: one graph per buffer
-        if (!A.graph_rev[b]) {
-          cudaGraph_t g = nullptr;
-          SFG_CUDA(cudaStreamBeginCapture(rs, cudaStreamCaptureModeThreadLocal));
-          reverse_segment(h, b, k1 - k0, false, rs);
-          SFG_CUDA(cudaStreamEndCapture(rs, &g));
-          SFG_CUDA(cudaGraphInstantiate(&A.graph_rev[b], g, 0));
-          cudaGraphDestroy(g);
-        }
+        if (!A.graph_rev[b])
+          A.graph_rev[b] = capture_graph(rs, [&]() { reverse_segment(h, b, k1 - k0, false, rs); });
         SFG_CUDA(cudaGraphLaunch(A.graph_rev[b], rs));
       } else {
         reverse_segment(h, b, k1 - k0, c + 1 == A.ncheck, rs);

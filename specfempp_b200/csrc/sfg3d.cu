@@ -209,6 +209,7 @@ int guarded(sfg_handle3d *h, F &&fn) {
   try {
     return fn();
   } catch (const sfg3::CudaError &ex) {
+    cudaGetLastError();       // reported here, not by the next handle's call
     h->err = ex.what();
     return SFG_ERR_CUDA;
   } catch (const std::exception &ex) {
@@ -523,12 +524,19 @@ cudaGraphExec_t capture(sfg_handle3d *h, int n, bool last_predicts, int par) {
   const int save = h->par;
   h->par = par;
   SFG3_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  for (int i = 0; i < n; ++i) launch_step(h, h->stream, i + 1 < n || last_predicts);
-  SFG3_CUDA(cudaStreamEndCapture(h->stream, &g));
+  try {
+    for (int i = 0; i < n; ++i) launch_step(h, h->stream, i + 1 < n || last_predicts);
+  } catch (...) {   // while a capture is open, the thread may not allocate
+    h->par = save;
+    if (cudaStreamEndCapture(h->stream, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+    throw;
+  }
   h->par = save;
+  SFG3_CUDA(cudaStreamEndCapture(h->stream, &g));
   cudaGraphExec_t ex = nullptr;
-  SFG3_CUDA(cudaGraphInstantiate(&ex, g, 0));
+  const cudaError_t rc = cudaGraphInstantiate(&ex, g, 0);
   cudaGraphDestroy(g);
+  SFG3_CUDA(rc);
   return ex;
 }
 

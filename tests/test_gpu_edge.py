@@ -149,3 +149,37 @@ def test_given_start_time(sfg_lib, oracle_lib):
     late = sfg.Simulation2D(w.mesh, dt=w.dt, nstep=900, start_time=-0.01)
     with pytest.raises(sfg.SfgError, match="start time"):
         late.set_sources(srcs)
+
+
+def test_refused_launch_stays_with_its_handle(sfg_lib):
+    """More shots than a grid has tiles for: the handle reports the refused
+    launch, and the handles made before and after it in the same thread run
+    as if it had not been there."""
+    from specfempp_b200 import meshgen, sfg
+
+    def handle():
+        w = meshgen.elastic_psv_80x60(nstep=60)
+        sim = sfg.Simulation2D(w.mesh, dt=w.dt, nstep=60)
+        sim.set_sources([sfg.Source(x=2000.0, z=1500.0, f0=40.0, factor=1e10)])
+        sim.set_receivers([2050.0], [1500.0])
+        sim.initialize()
+        return sim
+
+    ref = handle()
+    ref.run(60)
+    before = handle()
+    mesh = meshgen.structured_mesh(1, 1, 0.0, 50.0, 0.0, 50.0, np.zeros(1, np.int32),
+                                   [(meshgen.ELASTIC, 2300.0, 3000.0, 1730.0)])
+    many = sfg.Simulation2D(mesh, dt=4e-4, nstep=1, nshots=32 * 65535 + 1, kernel_variant=4)
+    many.set_sources([sfg.Source(x=20.0, z=30.0, f0=40.0, factor=1e10)])
+    many.set_receivers([25.0], [25.0])
+    with pytest.raises(sfg.SfgError, match="invalid configuration"):
+        many.initialize()
+        many.run(1)
+    before.run(60)
+    after = handle()
+    after.run(60)
+    assert np.abs(ref.seismograms()).max() > 0
+    for s in (before, after):
+        assert np.array_equal(s.seismograms(), ref.seismograms())
+    many.close()
