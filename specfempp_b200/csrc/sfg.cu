@@ -309,6 +309,10 @@ int guarded(sfg_handle *h, F &&fn) {
   }
 }
 
+// The handle's streams do not wait for the legacy stream, where zero fills and
+// copies from pageable memory run: those are finished here before they start.
+void uploads_done() { SFG_CUDA(cudaStreamSynchronize(nullptr)); }
+
 // Graph of what `work` launches on s.  A launch that is refused ends the
 // capture too: while one is open, the thread may not allocate.
 template <typename F>
@@ -1821,6 +1825,7 @@ int sfg_set_sources(sfg_handle *h, int nsrc, const sfg_source2d *src) {
       put(h->d_src_arr2, a.src_arr2);
       put(h->d_stf, a.stf);
       refresh_tile_records(h);
+      uploads_done();
       h->adj.forward_done = false;
     }
     return int(SFG_OK);
@@ -1949,6 +1954,7 @@ int sfg_initialize(sfg_handle *h) {
     if (h->tile_ok) upload_tiles(h);
     h->btile_ok = compute_btile_ok(h);
     if (h->btile_ok) upload_btiles(h);
+    uploads_done();
     autotune(h);
     h->graph_steps = std::max(1, h->opt.steps_per_graph);
     recapture(h);
@@ -2464,6 +2470,7 @@ int sfg_set_model2d(sfg_handle *h, const float *rho, const float *kappa, const f
         SFG_CUDA(cudaMemcpy(h->adj.st_c, c1.data(), c1.size() * sizeof(float), cudaMemcpyHostToDevice));
       if (h->adj2.st_c && !c2.empty())
         SFG_CUDA(cudaMemcpy(h->adj2.st_c, c2.data(), c2.size() * sizeof(float), cudaMemcpyHostToDevice));
+      uploads_done();
       h->adj.forward_done = false;
     }
     return int(SFG_OK);
@@ -2713,6 +2720,7 @@ void adjoint_alloc(sfg_handle *h, int nstep, int interval) {
   if (cpl && !A2.lu) adj_medium_init(h, A2, h->ac, h->asmb.ac, SFG_MEDIUM_ACOUSTIC);
   adj_write_record(A, D);
   if (cpl) adj_write_record(A2, h->ac);
+  uploads_done();
   auto recorded = [&](int mode, int nsteps, bool last_predicts) {
     struct Off {
       int &mode;
@@ -3032,7 +3040,9 @@ int sfg_adjoint_gradient(sfg_handle *h, const float *seis_grad, float *grad_rho,
       SFG_CUDA(cudaStreamSynchronize(s));
       if (A.rstream) SFG_CUDA(cudaStreamSynchronize(A.rstream));
       if (A.gtab) cudaFree(A.gtab);
-      A.gtab = dalloc<float>(ng);
+      A.gtab = nullptr;
+      A.gtab_cap = 0;
+      SFG_CUDA(cudaMalloc(&A.gtab, ng * sizeof(float)));   // filled below, on s
       A.gtab_cap = ng;
       for (cudaGraphExec_t &g : A.graph_rev)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }

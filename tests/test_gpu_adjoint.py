@@ -673,3 +673,37 @@ def test_refused_model_leaves_the_handle_as_it_was(sfg_lib):
         out.append(sim.adjoint_gradient(weights))
     for x, y in zip(*out):
         assert np.abs(x).max() > 0 and np.array_equal(x, y)
+
+
+def test_gradient_on_a_busy_device(sfg_lib):
+    """A fresh handle's first gradient while other work fills the device, so
+    that zero fills and copies on one stream and kernels on another run in any
+    order that nothing forbids: the same bits as on an idle device."""
+    import torch
+    from specfempp_b200 import meshgen
+    w = meshgen.elastic_psv_80x60(nstep=200)
+    model = base_model(w.mesh)
+    weights = np.random.default_rng(6).standard_normal((NSTEP, len(w.rec_x), 2)).astype(np.float32)
+    side = torch.cuda.Stream()
+    a = torch.randn(8192, 8192, device="cuda", dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+
+    def load():
+        with torch.cuda.stream(side):
+            for _ in range(40):
+                a @ a
+
+    out = []
+    for busy in (False, True, True, True):
+        sim = setup(w)
+        if busy:
+            load()
+        sim.set_model(*[m.astype(np.float32) for m in model])
+        sim.forward_checkpointed(NSTEP, 50)
+        if busy:
+            load()
+        out.append(sim.adjoint_gradient(weights))
+        torch.cuda.synchronize()
+    for got in out[1:]:
+        for x, y in zip(got, out[0]):
+            assert np.abs(y).max() > 0 and np.array_equal(x, y)
