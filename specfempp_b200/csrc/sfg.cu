@@ -581,6 +581,22 @@ sfg::dev::BatchArgs batch_args(sfg_handle *h, const DevMedium &el, const int *st
   return B;
 }
 
+// Shared memory that the thread form may ask for: the attribute belongs to the
+// function, not to the handle, so it is set once, to the most a launch needs
+// (two lanes an element), never to the present launch's need.
+template <int NC, int GEO, int MAT>
+void bt_attribute() {
+  SFG_CUDA(cudaFuncSetAttribute(sfg::dev::k_stiffness_batched_t<NC, GEO, MAT>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                sfg::dev::bt_words<GEO, MAT>() * (sfg::dev::BT_THREADS / 2) * sfg::dev::NP *
+                                    int(sizeof(float))));
+}
+
+void bt_attributes() {
+  bt_attribute<2, 1, 1>(); bt_attribute<2, 1, 0>(); bt_attribute<2, 0, 1>(); bt_attribute<2, 0, 0>();
+  bt_attribute<1, 1, 1>(); bt_attribute<1, 1, 0>(); bt_attribute<1, 0, 1>(); bt_attribute<1, 0, 0>();
+}
+
 void launch_stiffness_batched(sfg_handle *h, const DevMedium &el, const int *step, cudaStream_t s,
                               int variant) {
   sfg::dev::BatchArgs B{};
@@ -629,8 +645,8 @@ void launch_stiffness_batched(sfg_handle *h, const DevMedium &el, const int *ste
     const dim3 grid((el.nspec + ne - 1) / ne, (el.S + 31) / 32);
     auto go = [&](auto kern, int words) {
       const int smem = words * ne * sfg::dev::NP * int(sizeof(float));
-      SFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       kern<<<grid, sfg::dev::BT_THREADS, smem, s>>>(B, G);
+      SFG_CUDA(cudaGetLastError());
     };
     const bool geo = h->asmb.el.row.straight, mat = h->asmb.el.row.matconst;
     auto pick = [&](auto nc) {
@@ -1955,6 +1971,7 @@ int sfg_initialize(sfg_handle *h) {
     h->btile_ok = compute_btile_ok(h);
     if (h->btile_ok) upload_btiles(h);
     uploads_done();
+    if (a.nshots > 1) bt_attributes();
     autotune(h);
     h->graph_steps = std::max(1, h->opt.steps_per_graph);
     recapture(h);

@@ -63,3 +63,39 @@ def test_batched_shot_matches_oracle(sfg_lib, oracle_lib):
         ref = runner.run(case, "f32", nthreads=1)["seis"][:, 0]
         assert np.abs(ref).max() > 0
         assert rel_l2(seis[s, :, 0], ref) <= 1e-5, (s, rel_l2(seis[s, :, 0], ref))
+
+
+def test_batched_handles_of_several_threads(sfg_lib):
+    """Threads launch the thread form (variant 4) on handles of different shot
+    counts, and so of different shared-memory needs, at the same time: no
+    launch is refused (the limit is the function's, shared by all)."""
+    import threading
+    from specfempp_b200 import meshgen, sfg
+    mesh = meshgen.structured_mesh(9, 7, 0.0, 900.0, 0.0, 700.0, np.zeros(7, np.int32),
+                                   [(meshgen.ELASTIC, 2300.0, 3000.0, 1730.0)], absorbing=("bottom",))
+    x, z = mesh.coorg[:, 0], mesh.coorg[:, 1]
+    mesh.coorg = mesh.coorg + np.stack([0 * x, 9.0 * np.sin(x / 100.0) * z / 700.0], 1)
+    f = 1.0 + 0.05 * np.random.default_rng(8).uniform(-1, 1, (3, mesh.nspec, 25)).astype(np.float32)
+    pts = dict(zip(("point_rho", "point_vp", "point_vs"), (f.T * [2300.0, 3000.0, 1730.0]).T.astype(np.float32)))
+    sims = []
+    for shots in (2, 33) * 4:     # 57,600 and 3,600 bytes a block
+        s = sfg.Simulation2D(mesh, dt=4e-4, nstep=10, nshots=shots, kernel_variant=4, **pts)
+        s.set_sources([sfg.Source(x=400.0, z=300.0, f0=20.0, factor=1e10, shot=k) for k in range(shots)])
+        s.set_receivers([500.0], [400.0])
+        s.initialize()
+        sims.append(s)
+    errors = []
+
+    def work(s):
+        try:
+            for _ in range(60):
+                s.time_kernel(0, 300)
+                s.time_kernel(0, 5, 16)
+        except sfg.SfgError as e:
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(s,)) for s in sims]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
