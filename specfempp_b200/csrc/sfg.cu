@@ -1059,6 +1059,15 @@ void refresh_tile_records(sfg_handle *h) {
   }
 }
 
+// A tile kernel may use all the shared memory of a block.  The limit belongs
+// to the function, so it is not one handle's own need.
+template <typename K>
+void tile_attribute(K kern) {
+  cudaFuncAttributes fa{};
+  SFG_CUDA(cudaFuncGetAttributes(&fa, kern));
+  SFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - int(fa.sharedSizeBytes)));
+}
+
 // Device data of the fused tile kernel (after the receivers are known) and
 // its shared-memory layout.  Clears h->tile_ok when the layout does not fit.
 void upload_tiles(sfg_handle *h) {
@@ -1156,7 +1165,7 @@ void upload_tiles(sfg_handle *h) {
     h->tile_smem = L.acc_off + 16 * ncolors(D) * D.ncomp * L.kcap;
     if (h->tile_smem > 227 * 1024) { h->tile_ok = false; return; }
     auto kern = D.ncomp == 1 ? dv::k_tile_b<1> : dv::k_tile_b<2>;
-    SFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, h->tile_smem));
+    tile_attribute(kern);
     int nb = 0;
     SFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, dv::TILE_P, h->tile_smem));
     h->tile_blocks_per_sm = std::max(nb, 1);
@@ -1183,7 +1192,7 @@ void upload_tiles(sfg_handle *h) {
   h->tile_smem = L.acc_off + 4 * accw;
   if (h->tile_smem > 227 * 1024) { h->tile_ok = false; return; }
   auto kern = h->el.ncomp == 1 ? dv::k_tile<1> : dv::k_tile<0>;
-  SFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, h->tile_smem));
+  tile_attribute(kern);
   int nb = 0;
   SFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, dv::TILE_P, h->tile_smem));
   h->tile_blocks_per_sm = std::max(nb, 1);
