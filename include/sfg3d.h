@@ -4,8 +4,8 @@
  * 8-node hexahedra (arbitrary control-node coordinates), isotropic elastic
  * media given per GLL point, force and moment-tensor sources, receivers, the
  * Newmark time loop captured in CUDA graphs.  Status codes and sfg_options
- * are those of sfg.h (elements_per_block, 1, 2, 4, 6 or 8, fixes the layers of
- * elements that a block of the layer kernel marches through, or the least that
+ * are those of sfg.h (elements_per_block, 1, 2, 4, 6, 8 or 16, fixes the layers
+ * of elements that a block of the layer kernel marches through, or the least that
  * needs no more than 65,535 blocks in z; 0 lets the autotuner choose; all give
  * the same bits; kernel_variant is ignored).
  *

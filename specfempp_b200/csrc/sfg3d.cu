@@ -468,9 +468,9 @@ void setup_sources(sfg_handle3d *h) {
   }
 }
 
-// Layers a block marches: the caller's elements_per_block (1, 2, 4, 6 or 8)
-// or the autotuner's pick; no choice changes a bit.
-bool valid_layers(int e) { return e == 1 || e == 2 || e == 4 || e == 6 || e == 8; }
+// Layers a block marches: the caller's elements_per_block (1, 2, 4, 6, 8 or
+// 16) or the autotuner's pick (6 on request only); no choice changes a bit.
+bool valid_layers(int e) { return e == 1 || e == 2 || e == 4 || e == 6 || e == 8 || e == 16; }
 
 template <typename... P, typename... A>
 void launch_pdl(bool dependent, void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A &&...args) {

@@ -202,3 +202,21 @@ def test_3d_more_layers_than_a_grid_dimension(sfg_lib, epb):
         s.run(3)
     u = a.field("displacement")
     assert np.abs(u).max() > 0 and np.array_equal(u, b.field("displacement"))
+
+
+def test_3d_sixteen_layers_a_block(sfg_lib):
+    """What the tuner can pick can be asked for: 16 layers a block on a mesh
+    of 19 (a partial last march), the same bits as one layer; a handle made
+    with what another reports runs the same shape."""
+    shape = (5, 3, 19)
+    one, many = (small_handle(epb=e, shape=shape) for e in (1, 16))
+    assert many.info().elements_per_block == 16
+    tuned = small_handle(shape=shape)
+    again = small_handle(epb=tuned.info().elements_per_block, shape=shape)
+    assert again.info().elements_per_block == tuned.info().elements_per_block
+    for s in (one, many, tuned, again):
+        s.run(60)
+    assert np.abs(one.field("displacement")).max() > 0
+    for s in (many, tuned, again):
+        assert np.array_equal(one.seismograms(), s.seismograms())
+        assert np.array_equal(one.field("displacement"), s.field("displacement"))
