@@ -60,6 +60,12 @@ struct DevMem {
     SFG3_CUDA(cudaMemset(d, 0, n * sizeof(T)));
     return d;
   }
+  template <typename T>
+  void release(T *p, size_t n) {      // of n values
+    ptrs.erase(std::find(ptrs.begin(), ptrs.end(), static_cast<void *>(p)));
+    bytes -= n * sizeof(T);
+    cudaFree(p);
+  }
   ~DevMem() {
     for (void *p : ptrs) cudaFree(p);
   }
@@ -769,8 +775,7 @@ int sfg3d_initialize(sfg_handle3d *h) {
                                    sfg3::dev::L3_SMEM));
     SFG3_CUDA(cudaFuncSetAttribute(sfg3::dev::k_layer3d<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    sfg3::dev::L3_SMEM));
-    // the tiles' parts of shared points: sized for the shortest march tried
-    // (the grid's second dimension holds at most 65,535 of them)
+    // the marches of a mesh are the grid's second dimension: at most 65,535
     const int least = (h->nez + 65534) / 65535;
     std::vector<int> cand;
     if (valid_layers(h->opt.elements_per_block)) cand = {std::max(h->opt.elements_per_block, least)};
@@ -780,9 +785,11 @@ int sfg3d_initialize(sfg_handle3d *h) {
     if (cand.empty()) cand.push_back(least);
     const size_t ntile = size_t(A.nbx) * A.nby;
     A.rim = m.zeros<float>(ntile * A.NZ * sfg3::dev::NEDGE * 3);
-    const size_t parts = ntile * size_t((h->nez + cand[0] - 1) / cand[0]) * sfg3::dev::NCOL * 3;
-    A.lower = m.zeros<float>(parts);
-    A.upper = m.zeros<float>(parts);
+    // the tiles' parts of shared points: sized for the shortest march tried,
+    // then for the one kept (128x128x64: 481 MB, then 30 MB)
+    auto parts = [&](int L) { return ntile * size_t((h->nez + L - 1) / L) * sfg3::dev::NCOL * 3; };
+    A.lower = m.zeros<float>(parts(cand[0]));
+    A.upper = m.zeros<float>(parts(cand[0]));
     SFG3_CUDA(cudaDeviceSynchronize());
     h->layers = cand[0];
     if (cand.size() > 1) {
@@ -803,6 +810,13 @@ int sfg3d_initialize(sfg_handle3d *h) {
         if (t < best) { best = t; pick = L; }
       }
       h->layers = pick;
+      if (pick != cand[0]) {
+        for (float **p : {&A.lower, &A.upper}) {
+          m.release(*p, parts(cand[0]));
+          *p = m.zeros<float>(parts(pick));
+        }
+        SFG3_CUDA(cudaDeviceSynchronize());
+      }
     }
     for (int p = 0; p < 2; ++p) {
       h->graph_k[p] = capture(h, h->graph_steps, true, p);

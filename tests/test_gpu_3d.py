@@ -220,3 +220,12 @@ def test_3d_sixteen_layers_a_block(sfg_lib):
     for s in (many, tuned, again):
         assert np.array_equal(one.seismograms(), s.seismograms())
         assert np.array_equal(one.field("displacement"), s.field("displacement"))
+
+
+@pytest.mark.parametrize("shape", [(5, 3, 4), (48, 48, 32)])
+def test_3d_scratch_is_sized_for_the_march_in_use(sfg_lib, shape):
+    """A tuned handle holds no more device memory than one made with the
+    tuner's choice."""
+    tuned = small_handle(shape=shape).info()
+    fixed = small_handle(epb=tuned.elements_per_block, shape=shape).info()
+    assert tuned.device_bytes == fixed.device_bytes
