@@ -558,7 +558,11 @@ void resume(sfg_handle3d *h) {
 
 // n steps that end on the next step's predictor.
 void run_fused(sfg_handle3d *h, int n) {
-  for (; n >= h->graph_steps; n -= h->graph_steps) SFG3_CUDA(cudaGraphLaunch(h->graph_k[h->par], h->stream));
+  for (; n >= h->graph_steps; n -= h->graph_steps) {
+    cudaGraphExec_t &g = h->graph_k[h->par];
+    if (!g) g = capture(h, h->graph_steps, true, h->par);
+    SFG3_CUDA(cudaGraphLaunch(g, h->stream));
+  }
   for (; n > 0; --n) {
     SFG3_CUDA(cudaGraphLaunch(h->graph_1[h->par], h->stream));
     h->par ^= 1;
@@ -818,8 +822,9 @@ int sfg3d_initialize(sfg_handle3d *h) {
         SFG3_CUDA(cudaDeviceSynchronize());
       }
     }
+    // graph_k of the second buffer when a run first starts from it
+    h->graph_k[0] = capture(h, h->graph_steps, true, 0);
     for (int p = 0; p < 2; ++p) {
-      h->graph_k[p] = capture(h, h->graph_steps, true, p);
       h->graph_1[p] = capture(h, 1, true, p);
       h->graph_e[p] = capture(h, 1, false, p);
     }
