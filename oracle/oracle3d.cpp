@@ -125,6 +125,8 @@ struct Sim3D {
   T hpw[NG][NG];   // hp[l][i] * w[l] rounded once (device evaluation order)
   std::vector<int> ibool;                           // [nspec][125]
   std::vector<T> g9, jac, c0, mu;                   // g9: [nspec][125][9]
+  // device order: |J| folded in, g9 |J|, c0 / |J|, mu / |J|, each rounded once
+  std::vector<T> g9j, c0j, muj;
   std::vector<T> u, v, a, minv;                     // [nglob][3]
   struct Face { int e, q; T n[3]; T rvp, rvs, w; };   // one absorbing face point
   std::vector<Face> faces;
@@ -160,6 +162,7 @@ struct Sim3D {
   void setup() {
     const size_t nloc = size_t(nspec) * NP3;
     ibool.resize(nloc); g9.resize(nloc * 9); jac.resize(nloc); c0.resize(nloc); mu.resize(nloc);
+    if (in.device_order) { g9j.resize(nloc * 9); c0j.resize(nloc); muj.resize(nloc); }
     std::vector<double> mass(size_t(nglob), 0.0);
     for (int e = 0; e < nspec; ++e) {
       double cn[8][3];
@@ -181,6 +184,12 @@ struct Sim3D {
             const double kappa = rho * (vp * vp - 4.0 / 3.0 * vs * vs);
             c0[p] = T(kappa + 4.0 / 3.0 * m);
             mu[p] = T(m);
+            if (in.device_order) {
+              for (int k = 0; k < 3; ++k)
+                for (int j = 0; j < 3; ++j) g9j[p * 9 + k * 3 + j] = T(G.inv[k][j] * G.jac);
+              c0j[p] = T((kappa + 4.0 / 3.0 * m) / G.jac);
+              muj[p] = T(m / G.jac);
+            }
             mass[size_t(ibool[p])] += rho * wd[ix] * wd[iy] * wd[iz] * G.jac;
           }
     }
@@ -364,10 +373,13 @@ struct Sim3D {
             }
             dxi[c][0] = s0; dxi[c][1] = s1; dxi[c][2] = s2;
           }
-          const T *gi = &g9[p * 9];
-          // device order: the map, the normal stresses and F as FMA chains,
-          // as the CUDA element kernels compute them (dot3 / stress3)
+          // device order: the map, the normal stresses and F as FMA chains on
+          // the folded words, as the CUDA layer kernel computes them (dot3 /
+          // stress3; on a mesh of boxes along the axes the chains' other terms
+          // are zero).  It sums a point's contributions by tiles, this oracle
+          // by elements.
           const bool dv = in.device_order;
+          const T *gi = dv ? &g9j[p * 9] : &g9[p * 9];
           auto dot3 = [dv](T a0, T b0, T a1, T b1, T a2, T b2) {
             return dv ? T(std::fma(a2, b2, std::fma(a1, b1, a0 * b0))) : a0 * b0 + a1 * b1 + a2 * b2;
           };
@@ -375,7 +387,7 @@ struct Sim3D {
           for (int c = 0; c < 3; ++c)
             for (int j = 0; j < 3; ++j)
               du[c][j] = dot3(dxi[c][0], gi[0 * 3 + j], dxi[c][1], gi[1 * 3 + j], dxi[c][2], gi[2 * 3 + j]);
-          const T l2m = c0[p], m = mu[p], lam = l2m - T(2) * m;
+          const T l2m = dv ? c0j[p] : c0[p], m = dv ? muj[p] : mu[p], lam = l2m - T(2) * m;
           T sig[3][3];
           if (dv) {
             sig[0][0] = std::fma(l2m, du[0][0], lam * (du[1][1] + du[2][2]));
@@ -391,7 +403,8 @@ struct Sim3D {
           sig[1][2] = sig[2][1] = m * (du[1][2] + du[2][1]);
           for (int c = 0; c < 3; ++c)
             for (int k = 0; k < 3; ++k)
-              F[q][c][k] = jac[p] * dot3(sig[c][0], gi[k * 3 + 0], sig[c][1], gi[k * 3 + 1], sig[c][2], gi[k * 3 + 2]);
+              F[q][c][k] = (dv ? T(1) : jac[p]) *
+                           dot3(sig[c][0], gi[k * 3 + 0], sig[c][1], gi[k * 3 + 1], sig[c][2], gi[k * 3 + 2]);
         }
     T r[NP3][3];
     for (int iz = 0; iz < NG; ++iz)

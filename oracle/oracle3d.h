@@ -22,7 +22,9 @@ typedef struct OracleInput3D {
   double dt;
   int nstep;
   /* 0: the reference's evaluation order; 1: the device kernels' order (the
-   * 5-term contractions as fused multiply-adds, hprime * w rounded once) */
+   * 5-term contractions, the derivative map, the stress and F as fused
+   * multiply-adds, hprime * w rounded once, |J| folded into the metric terms
+   * and the moduli) */
   int device_order;
 } OracleInput3D;
 
