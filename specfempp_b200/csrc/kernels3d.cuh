@@ -15,8 +15,10 @@
 //   contributions are then summed per unique point in shared memory (x
 //   neighbours, then y, then the layer below) and every point that no other
 //   tile touches is finished at once: a = sum * M^-1, Newmark corrector, next
-//   predictor (newmark.tpp:10-128).  Only the tile's shared points (a fifth of
-//   all) pass through memory.
+//   predictor (newmark.tpp:10-128).  Only the tile's shared points pass through
+//   memory: 23 of an inner tile's 128 columns, and of the others the plane
+//   between two marches, 1 - (105/128) (1 - 1/(4 L)) of all points for marches
+//   of L layers (38% for one, 28% for two, 23% for four).
 // * Finish kernel (k_finish3d): sums the tiles' parts of the shared points in
 //   tile order (across a z boundary of two blocks of one tile: lower plus
 //   upper first), finishes them, and takes the receivers that read only the
@@ -31,8 +33,8 @@
 // Why this split: a kernel per element with its contributions in memory moves
 // 12 B a contribution out and back (3.9 contributions' worth a point counting
 // index arrays, 185 B a point and step); marching tiles move 60 B of fields and
-// M^-1 and 15.5 B of material a point plus the shared fifth.  The metric terms
-// are folded (|J| into grad xi, 1/|J| into the moduli), which drops the
+// M^-1 and 15.5 B of material a point, and at the shared points the tiles' parts
+// out and back and the fields once more.  The metric terms are folded (|J| into grad xi, 1/|J| into the moduli), which drops the
 // Jacobian word and nine products a point; a mesh of boxes along the axes
 // (GEO 1, decided for the whole mesh at set-up) keeps three metric words an
 // element.
@@ -159,8 +161,6 @@ __device__ __forceinline__ void st_col(float *s, const Col &c) {
   for (int i = 0; i < 4; ++i)
     reinterpret_cast<float4 *>(s)[i] = make_float4(c.p[2 * i].x, c.p[2 * i].y, c.p[2 * i + 1].x, c.p[2 * i + 1].y);
 }
-template <int I>
-__device__ __forceinline__ float &cv(Col &c) { return I & 1 ? c.p[I >> 1].y : c.p[I >> 1].x; }
 __device__ __forceinline__ float cget(const Col &c, int i) { return i & 1 ? c.p[i >> 1].y : c.p[i >> 1].x; }
 __device__ __forceinline__ void cset(Col &c, int i, float v) {
   if (i & 1) c.p[i >> 1].y = v;
@@ -506,7 +506,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) k_layer3d(const __grid_consta
 }
 
 // One receiver by 128 threads (q = thread, red [3][128]): Lagrange
-// interpolation with a fixed-order tree sum.  mask: the types to take.
+// interpolation with a fixed-order tree sum.  late: the velocity and
+// acceleration types, else the displacement ones.
 __device__ __forceinline__ void receive3(const Step3Args &A, int rr, int q, float (*red)[128], bool on, bool late) {
   const int e = on ? A.rec_elem[rr] : 0;
   const int ex = e % A.nex, ey = (e / A.nex) % A.ney, ez = e / (A.nex * A.ney);

@@ -74,9 +74,8 @@ def test_3d_absorbing_moment_tensor_vs_oracle(sfg_lib, oracle_lib):
 
 
 def test_3d_launch_shapes_agree_and_deterministic(sfg_lib):
-    """Point form (1, 2, 4 elements per block) and column form (6, 8): the
-    same bits, seismograms and final field, with sources and absorbing
-    faces."""
+    """One to eight element layers a block: the same bits, seismograms and
+    final field, with sources and absorbing faces."""
     case = small_absorbing_case(nstep=120)
     s1, a = product3d(case, epb=1)
     _, b = product3d(case, epb=4)

@@ -52,14 +52,13 @@ def simulate(mesh, kind, nstep, variant, epb=0, points=None, nshots=1, types=Non
     return sim
 
 
-@pytest.mark.parametrize("kind", ["psv", "sh", "acoustic", "poro"])
 @pytest.mark.parametrize("nx,nz", [(3, 2), (33, 1), (16, 10), (13, 37)])
-@pytest.mark.parametrize("relief,varied", [(0.0, False), (0.0, True), (9.0, False), (9.0, True)])
+@pytest.mark.parametrize("kind,relief,varied", [
+    (kind, relief, varied) for kind in ("psv", "sh", "acoustic", "poro") for relief in (0.0, 9.0)
+    for varied in (False, True) if not (kind == "poro" and varied)])     # poroelastic: material constants only
 def test_row_form_keeps_the_bits(sfg_lib, kind, nx, nz, relief, varied):
     """Row form (both block sizes) against the colour passes: every
     specialisation, blocks that the mesh fills partly."""
-    if varied and kind == "poro":
-        pytest.skip("poroelastic media take material constants only")
     mesh = grid(kind, nx, nz, relief)
     points = None
     if varied:
@@ -75,6 +74,25 @@ def test_row_form_keeps_the_bits(sfg_lib, kind, nx, nz, relief, varied):
         assert sim.info().kernel_variant == 6
         assert np.array_equal(sim.seismograms(), a)
         assert np.array_equal(sim.field(med), u)
+
+
+@pytest.mark.parametrize("kind,shots", [("psv", 1), ("sh", 1), ("acoustic", 1), ("poro", 1), ("psv", 6), ("sh", 6)])
+def test_one_tilted_element_among_rectangles(sfg_lib, kind, shots):
+    """A mesh of rectangles whose corner node is moved by 2% of an element:
+    the element there is no rectangle, so the mesh takes the general kernels
+    (row form, or thread form of batched shots), and the bits are the colour
+    passes' and not those of the straight mesh."""
+    mesh = grid(kind, 17, 9, 0.0)
+    flat = simulate(mesh, kind, 400, 1, 16, nshots=shots)
+    corner = np.argmin(mesh.coorg.sum(1))
+    mesh.coorg = mesh.coorg.copy()
+    mesh.coorg[corner] += 1.0
+    ref, sim = (simulate(mesh, kind, 400, v, 16, nshots=shots) for v in (1, 6 if shots == 1 else 4))
+    med = "acoustic" if kind == "acoustic" else "elastic"
+    assert sim.info().kernel_variant == (6 if shots == 1 else 4)
+    assert np.array_equal(sim.seismograms(), ref.seismograms())
+    assert np.array_equal(sim.field(med), ref.field(med))
+    assert not np.array_equal(ref.field(med), flat.field(med))
 
 
 def test_model_class_change_under_captured_graphs(sfg_lib):
@@ -150,6 +168,33 @@ def test_reverse_row_form_keeps_the_bits(sfg_lib, relief, varied):
         out.append(sim.adjoint_gradient(weights))
     for x, y in zip(*out):
         assert np.abs(x).max() > 0 and np.array_equal(x, y)
+
+
+def test_3d_one_deformed_element_among_boxes(sfg_lib, oracle_lib):
+    """A mesh of boxes whose corner node is moved by 10%: the whole mesh takes
+    the general metric, within 1e-5 of the oracle FP32 (the straight mesh's
+    field is not)."""
+    from oracle import runner3d
+    from specfempp_b200 import meshgen, sfg3d
+    fields = []
+    for moved in (False, True):
+        mesh = meshgen.homogeneous_hex_mesh(5, 3, 2, (0, 300.0, 0, 180.0, -120.0, 0), 2300.0, 3000.0, 1700.0,
+                                            absorbing=(1, 0, 1, 1, 1, 0))
+        if moved:
+            mesh.nodes = mesh.nodes.copy()
+            mesh.nodes.reshape(-1, 3)[0] += (6.0, -4.0, 5.0)
+        src = [runner3d.Source3D(35.0, 30.0, -90.0, f0=45.0, factor=1e10, comp=(0.2, 1.0, -0.6, 0, 0, 0))]
+        rec = np.array([[70.0, 60.0, -60.0]])
+        sim = sfg3d.Simulation3D(mesh, dt=3e-4, nstep=150)
+        sim.set_sources(src)
+        sim.set_receivers(rec)
+        sim.initialize()
+        sim.run(150)
+        fields.append(sim.field())
+    ref = runner3d.run(runner3d.Case3D(mesh, src, rec, 3e-4, 150, ["displacement"]), "f32", nthreads=4,
+                       want_final=True)["final"]
+    assert rel_l2(fields[1], ref) <= 1e-5
+    assert rel_l2(fields[0], ref) > 1e-3
 
 
 @pytest.mark.parametrize("shape", [(1, 1, 1), (4, 2, 1), (5, 3, 2), (3, 5, 4), (9, 4, 3)])
