@@ -40,7 +40,9 @@
 // element.
 //
 // Measured, 48x48x32 boxes with moduli per point (4.8 M points): step 370 ->
-// 291 us; layer kernel 232 us (2 layers a block), finish kernel 52 us.
+// 291 us; layer kernel 232 us and finish kernel 64 us one after another (2
+// layers a block; they overlap in a step).  Deformed, general metric: step 406
+// us, layer kernel 349 us.
 // 13x11x9: 17.9 -> 17.3 us.  The layer kernel is bound by shared memory (its
 // wavefronts take 67% of the L1's cycles) and by the barriers of a layer at
 // two blocks a SM; three blocks at 80 registers spill and take 250 us.  The

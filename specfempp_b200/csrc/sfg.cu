@@ -760,7 +760,7 @@ sfg::dev::UpdateArgs update_args(sfg_handle *h, const DevMedium &D, const DevMed
   // acoustic chi_dd feeds the elastic coupling term; the last step of a run
   // keeps the acceleration for the predictor that resumes the next run.  The
   // gather form stores, within a run, only the interface points' chi_dd
-  // (500x250: 8 MB less a step, update 11.3 -> 11.0 us)
+  // (500x250: 8 MB less a step, update 13.0 -> 12.4 us, step 35.7 -> 34.4)
   const bool keep_a = !predict || h->opt.store_acceleration;
   U.a_store = (medium == SFG_MEDIUM_ACOUSTIC || keep_a) ? D.a : nullptr;
   U.a_n = keep_a ? int(D.values()) / D.ncomp : D.a_read;
