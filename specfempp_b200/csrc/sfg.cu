@@ -2469,6 +2469,7 @@ int sfg_set_model2d(sfg_handle *h, const float *rho, const float *kappa, const f
     const bool ac_src = h->have_sources && h->asmb.ac.nspec > 0 && h->asmb.nsrc > 0;
     if (ac_src) sfg::set_sources2d(h->mesh, h->asmb, h->sources);
     if (h->initialized) {
+      SFG_CUDA(cudaStreamSynchronize(h->stream));    // a run in flight keeps its model
       if (ac_src)
         SFG_CUDA(cudaMemcpy(h->d_src_arr, h->asmb.src_arr.data(), h->asmb.src_arr.size() * sizeof(float),
                             cudaMemcpyHostToDevice));

@@ -129,6 +129,23 @@ def test_model_class_change_under_captured_graphs(sfg_lib):
     assert np.array_equal(sim.seismograms(), run(simulate(mesh, "psv", 80, 3, 8), models[0])[0])
 
 
+def test_model_change_waits_for_the_run_in_flight(sfg_lib):
+    """sfg_run returns before the device is done; a model set at once does not
+    touch that run's steps."""
+    from specfempp_b200 import adjoint
+    mesh = grid("psv", 60, 50, 0.0)
+    rho, vp, vs = (a[mesh.kmato][:, None] * np.ones((1, 25)) for a in (mesh.mat_rho, mesh.mat_vp, mesh.mat_vs))
+    other = [m.astype(np.float32) for m in (1.2 * rho, *adjoint.moduli(1.2 * rho, 0.9 * vp, 0.9 * vs))]
+    ref = simulate(mesh, "psv", 3000, 6, 32)
+    want = ref.seismograms(), ref.field("elastic")
+    sim = simulate(mesh, "psv", 3000, 6, 32)
+    sim.reset()
+    sim.run(3000)
+    sim.set_model(*other)
+    assert np.abs(want[0]).max() > 0
+    assert np.array_equal(sim.seismograms(), want[0]) and np.array_equal(sim.field("elastic"), want[1])
+
+
 @pytest.mark.parametrize("kind", ["psv", "sh"])
 @pytest.mark.parametrize("nshots", [2, 3, 6, 16, 20, 33])
 @pytest.mark.parametrize("relief,varied", [(0.0, False), (7.0, True), (0.0, True)])
