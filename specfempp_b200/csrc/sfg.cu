@@ -592,9 +592,18 @@ void bt_attribute() {
                                     int(sizeof(float))));
 }
 
-void bt_attributes() {
-  bt_attribute<2, 1, 1>(); bt_attribute<2, 1, 0>(); bt_attribute<2, 0, 1>(); bt_attribute<2, 0, 0>();
-  bt_attribute<1, 1, 1>(); bt_attribute<1, 1, 0>(); bt_attribute<1, 0, 1>(); bt_attribute<1, 0, 0>();
+// The kernels that a handle can launch: its material class may change.
+void bt_attributes(int ncomp, bool straight) {
+  auto both = [&](auto nc, auto geo) {
+    bt_attribute<decltype(nc)::value, decltype(geo)::value, 0>();
+    bt_attribute<decltype(nc)::value, decltype(geo)::value, 1>();
+  };
+  auto comp = [&](auto nc) {
+    if (straight) both(nc, std::integral_constant<int, 1>{});
+    else both(nc, std::integral_constant<int, 0>{});
+  };
+  if (ncomp == 2) comp(std::integral_constant<int, 2>{});
+  else comp(std::integral_constant<int, 1>{});
 }
 
 void launch_stiffness_batched(sfg_handle *h, const DevMedium &el, const int *step, cudaStream_t s,
@@ -1980,7 +1989,7 @@ int sfg_initialize(sfg_handle *h) {
     h->btile_ok = compute_btile_ok(h);
     if (h->btile_ok) upload_btiles(h);
     uploads_done();
-    if (a.nshots > 1) bt_attributes();
+    if (a.nshots > 1) bt_attributes(h->el.ncomp, a.el.row.straight);
     autotune(h);
     h->graph_steps = std::max(1, h->opt.steps_per_graph);
     recapture(h);
